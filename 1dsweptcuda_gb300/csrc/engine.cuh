@@ -509,6 +509,23 @@ __device__ __forceinline__ void euler_level_warp(const Params<T> &p, T *rows, in
     }
 }
 
+// The interface (b-1, b) of a level on the FP64 pipe alone (a flagged lane of
+// eu_iface_q): F and S as eu_iface forms them.
+template <typename T>
+__device__ __noinline__ void euler_iface_pipe(const Params<T> &p, const T *src, const T *D, T *F, T *S, int L, int b) {
+    Q3<T> c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) c[k] = q3(src[b - 2 + k], src[L + b - 2 + k], src[2 * L + b - 2 + k]);
+    Q3<T> f, g;
+    eu_iface(p, c[0], c[1], c[2], c[3], D[b - 1], D[b], D[b + 1], f, g);
+    F[b] = f.x;
+    F[L + b] = f.y;
+    F[2 * L + b] = f.z;
+    S[b] = g.x;
+    S[L + b] = g.y;
+    S[2 * L + b] = g.z;
+}
+
 // Euler sub-step over tile cells [lo, hi) of a swept tile, every interface
 // computed once, in three passes of the whole block through shared memory
 // (xs: kEulerIfaceArrays rows of L values after the tile rows):
@@ -543,7 +560,12 @@ __device__ __forceinline__ void euler_level_tile(const Params<T> &p, T *rows, in
 #pragma unroll
         for (int k = 0; k < 4; ++k) c[k] = q3(src[b - 2 + k], src[L + b - 2 + k], src[2 * L + b - 2 + k]);
         Q3<T> f, g;
-        eu_iface(p, c[0], c[1], c[2], c[3], D[b - 1], D[b], D[b + 1], f, g);
+        uint32_t bad = 0;
+        eu_iface_q(p, c[0], c[1], c[2], c[3], D[b - 1], D[b], D[b + 1], f, g, bad);
+        if (bad) {
+            euler_iface_pipe(p, src, D, F, S, L, b);
+            continue;
+        }
         F[b] = f.x;
         F[L + b] = f.y;
         F[2 * L + b] = f.z;
@@ -836,6 +858,27 @@ __global__ void __launch_bounds__(Scheme<P, T>::CMAXT) k_classic(const Params<T>
 // Classic Euler sub-step with shared interfaces (the warp scheme above over
 // the whole domain, 29 cells per warp).  Cells 0 and nx-1
 // hold the Dirichlet states (classicEuler, Euler1D_SweptShared.cu:400-426).
+// The interface of cells q-1 and q (q clamped as below) on the FP64 pipe alone
+// (a flagged lane): F and S together.
+template <typename T>
+struct IfaceTerms {
+    Q3<T> F, S;
+};
+template <typename T>
+__device__ __noinline__ IfaceTerms<T> classic_iface_pipe(const Params<T> &p, const V4<T> *__restrict__ in, int64_t b, T D,
+                                                         T D1, T D2) {
+    Q3<T> c[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        int64_t q = b - 2 + k;
+        q = q < 0 ? 0 : (q >= p.nx ? p.nx - 1 : q);
+        const V4<T> v = in[q];
+        c[k] = q3(v.x, v.y, v.z);
+    }
+    IfaceTerms<T> t;
+    eu_iface(p, c[0], c[1], c[2], c[3], D, D1, D2, t.F, t.S);
+    return t;
+}
 template <typename T>
 __global__ void __launch_bounds__(256) k_classic_euler(const Params<T> p, const V4<T> *__restrict__ in,
                                                        V4<T> *__restrict__ out, const int sub) {
@@ -853,7 +896,13 @@ __global__ void __launch_bounds__(256) k_classic_euler(const Params<T> p, const 
     const T D = (b - 1 == 0 || b - 2 == nx - 1) ? T(0) : eu_pdiff(c[0], c[1]);
     const T D1 = __shfl_down_sync(0xffffffffu, D, 1), D2 = __shfl_down_sync(0xffffffffu, D, 2);
     Q3<T> F, S;
-    eu_iface(p, c[0], c[1], c[2], c[3], D, D1, D2, F, S);
+    uint32_t bad = 0;
+    eu_iface_q(p, c[0], c[1], c[2], c[3], D, D1, D2, F, S, bad);
+    if (bad) {
+        const IfaceTerms<T> t = classic_iface_pipe(p, in, b, D, D1, D2);
+        F = t.F;
+        S = t.S;
+    }
     const Q3<T> Fr = shfl_down3(F, 1), Sr = shfl_down3(S, 1);
     if (lane >= kEulerCellsPerWarp || b >= nx) return;
     if (b == 0 || b == nx - 1) {

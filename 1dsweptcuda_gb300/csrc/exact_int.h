@@ -71,6 +71,16 @@ SW_HD double mul_pow2(double x, double f, int k) {
     return f64_mul_pipe(x, f);
 }
 
+// The same with a flag instead of the fallback (see mul_int_fast below); a
+// zero is its own product.
+SW_HD double mul_pow2_fast(double x, int k, uint32_t &bad) {
+    const uint64_t b = f64_bits(x);
+    const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
+    const bool zero = (b << 1) == 0;
+    bad |= (uint32_t)!(zero || (e - 1u < 2046u && e + (uint32_t)k - 1u < 2046u));
+    return f64_from_bits(zero ? b : b + ((uint64_t)(int64_t)k << 52));
+}
+
 // x * 6.
 SW_HD double mul6(double x) {
     const uint64_t b = f64_bits(x);
@@ -93,17 +103,19 @@ SW_HD double mul6(double x) {
     return f64_mul_pipe(x, 6.0);
 }
 
-// ---- the general product on the integer pipe
+// ---- general products, quotients and square roots on the integer pipe
 //
-// mul_int_fast(x, y, bad) = x * y, rounded once (to nearest, ties to even), for
-// normal operands with a normal result (biased exponent at most 2045 before
-// rounding).  For anything else -- zeros, subnormals, infinities, NaNs, a
-// result near or outside the ends of the normal range -- it sets bad and the
-// result is meaningless: the caller recomputes that value with the FP64
-// multiply.  No FP64 instruction sits on its path, so none is issued: a
-// predicated-off FP64 instruction still holds the FP64 pipe, and a fallback
-// inside the product measured as slow as the multiply it replaces.
-// mul_int holds that fallback (host checks).
+// mul_int_fast(x, y, bad) = x * y, div_int_fast(x, y, bad) = x / y and
+// sqrt_int_fast(x, bad) = sqrt(x), each rounded once (to nearest, ties to
+// even), for normal operands with a normal result (biased exponent at most
+// 2045 before rounding); a division also takes a zero numerator.  For
+// anything else -- other zeros, subnormals, infinities, NaNs, a result near or
+// outside the ends of the normal range -- they set bad and the result is
+// meaningless: the caller recomputes that value with the FP64 instruction.
+// No FP64 instruction sits on their path, so none is issued: a predicated-off
+// FP64 instruction still holds the FP64 pipe, and a fallback inside the
+// product measured as slow as the multiply it replaces.
+// mul_int, div_int and sqrt_int hold that fallback (host checks).
 SW_HD uint32_t f64_hi(double x) {
 #if defined(__CUDA_ARCH__)
     return (uint32_t)__double2hiint(x);
@@ -187,6 +199,145 @@ SW_HD double mul_int_fast(double x, double y, uint32_t &bad) {
     const uint32_t e = (xh & kSignExp) + (yh & kSignExp) + (top << 20) - (1024u << 20);
     return round_pack(e, mh, ml, r, p0);
 }
+
+// ---- quotients
+//
+// A correctly rounded FP64 quotient in software on the FP64 pipe is eight or
+// more FP64 instructions (and a root as many) at 64 cycles or more of a
+// sub-partition's pipe each; here it is about 60 integer ones.  Euler FP64
+// swept (2^21 cells, tile 512; five to seven quotients and three roots per
+// interface): 1.48e9 -> 2.80e9 cell-updates/s.
+//
+// The reciprocal of the divisor's significand b in [1, 2) to 2^-29, as a
+// 32-bit fraction Y (Y / 2^32 <= 1 / b): the FP32 reciprocal approximation of
+// b's leading 24 bits (error below 2^-22; any seed that close will do), then
+// one Newton step y + y (1 - b y) in 32-bit integers.  bt holds b's leading 32
+// bits (bit 31 set); the step takes bt + 1 for b and rounds down, so Y never
+// exceeds the reciprocal.  Seed and step are the textbook ones; the quotient
+// below corrects every remaining error exactly.
+SW_HD float f32_rcp_seed(float x) {
+#if defined(__CUDA_ARCH__)
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return 1.0f / x;
+#endif
+}
+SW_HD float f32_rsqrt_seed(float x) {
+#if defined(__CUDA_ARCH__)
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+#else
+    return (float)(1.0 / __builtin_sqrt((double)x));
+#endif
+}
+SW_HD float f32_from_bits(uint32_t b) {
+#if defined(__CUDA_ARCH__)
+    return __uint_as_float(b);
+#else
+    float x;
+    memcpy(&x, &b, sizeof x);
+    return x;
+#endif
+}
+// y in (0.5, 1) as y * 2^23: the significand bits of 1 + y
+SW_HD uint32_t frac23(float y) {
+    const float z = 1.0f + y;
+#if defined(__CUDA_ARCH__)
+    return __float_as_uint(z) - 0x3f800000u;
+#else
+    uint32_t b;
+    memcpy(&b, &z, sizeof b);
+    return b - 0x3f800000u;
+#endif
+}
+SW_HD uint32_t rcp_newton(uint32_t bt, uint32_t y23) {
+    const uint32_t yh = y23 << 8;                  // y * 2^31
+    const uint64_t p = wide(bt, yh) + yh;          // (b + 2^-31) y * 2^62
+    const int32_t e = (int32_t)~(uint32_t)(p >> 12);  // (1 - b y) * 2^50, rounded down
+    const int32_t c = (int32_t)(((int64_t)(int32_t)yh * e) >> 32);
+    return (yh << 1) + (uint32_t)(c >> 17);
+}
+struct RcpInt {
+    uint32_t Y, n0, n1;  // the reciprocal; minus the significand (at bit 61) as two words
+    uint32_t hi;         // the divisor's high word
+};
+SW_HD float rcp_int_arg(double b) {  // b's significand in [1, 2), 24 bits (never 1, so that y < 1)
+    return f32_from_bits(0x3f800003u | (shl_hi(f64_lo(b), f64_hi(b), 3) & 0x007fffffu));
+}
+SW_HD RcpInt rcp_int_from(double b, float y) {
+    const uint32_t bh = f64_hi(b), bl = f64_lo(b);
+    const uint32_t bt = shl_hi(bl, bh, 11) | 0x80000000u;
+    const uint64_t n = 0ull - ((((uint64_t)(bt >> 2)) << 32) | (bl << 9));
+    return RcpInt{rcp_newton(bt, frac23(y)), (uint32_t)n, (uint32_t)(n >> 32), bh};
+}
+SW_HD RcpInt rcp_int(double b) { return rcp_int_from(b, f32_rcp_seed(rcp_int_arg(b))); }
+// a / b from b's reciprocal: long division of the significands A, B (at bit
+// 61) in two digits of 28 and 26 bits.  A digit is the remainder's leading 32
+// bits times Y, at most 2.5 (first) and 1.44 (second) below the true quotient,
+// so the remainders stay in [0, 2.5 B) -- below 2^64 -- and after the second
+// digit one comparison makes Q = floor(A / B * 2^54) exact.  The quotient of
+// two 53-bit significands is never halfway between two 53-bit numbers, so
+// rounding needs no sticky bit.
+SW_HD double div_int_with(double a, const RcpInt &b, uint32_t &bad) {
+    const uint32_t ah = f64_hi(a), al = f64_lo(a);
+    uint64_t R = ((uint64_t)((shl_hi(al, ah, 9) & 0x3fffffffu) | 0x20000000u) << 32) | (al << 9);
+    const uint64_t n = ((uint64_t)b.n1 << 32) | b.n0;
+    const uint32_t q1 = mulhi((uint32_t)(R >> 32), b.Y) >> 1;
+    R = (R << 28) + wide(q1, b.n0) + ((uint64_t)(q1 * b.n1) << 32);
+    const uint32_t q2 = mulhi((uint32_t)(R >> 32), b.Y) >> 3;
+    R = (R << 26) + wide(q2, b.n0) + ((uint64_t)(q2 * b.n1) << 32);
+    const uint64_t Q = wide(q1, 1u << 26) + q2 + (uint32_t)(R >= 0ull - n);
+    const uint32_t top = (uint32_t)(Q >> 54);
+    const uint64_t m = Q + top + 1u;
+    const uint32_t ml = shr_lo((uint32_t)m, (uint32_t)(m >> 32), top + 1u), mh = (uint32_t)(m >> 32) >> (top + 1u);
+    const uint32_t ea = (ah >> 20) & 0x7ffu, eb = (b.hi >> 20) & 0x7ffu;
+    const uint32_t sgn = (ah ^ b.hi) & 0x80000000u;
+    const uint32_t e = (ea - eb + 1021u + top) << 20;
+    const bool zero = ((ah << 1) | al) == 0;
+    // er = ea - eb + 1022 + top in 1 .. 2045
+    bad |= (uint32_t)!(eb - 1u < 2046u && (zero || (ea - 1u < 2046u && ea - eb + 1021u + top < 2045u)));
+    return f64_of(zero ? sgn : ((e + mh) | sgn), zero ? 0u : ml);
+}
+SW_HD double div_int_fast(double a, double b, uint32_t &bad) { return div_int_with(a, rcp_int(b), bad); }
+
+// ---- square roots
+//
+// With m = x 4^-k in [1, 4) and M = m 2^62: a 32-bit root s1 of M from the
+// FP32 reciprocal root y (biased down by 4 units of 2^-23, more than its error: s0 stays below the
+// root and nothing overflows)
+// and one correction by the remainder, s1 in (sqrt(M) - 2.1, sqrt(M) - 0.9];
+// then one digit d of 23 bits more, the remainder times 1 / (2 s1) with y
+// refined as a quotient's (s1 is the divisor).  s1 2^23 + d is S = floor(
+// sqrt(m) 2^54) or S - 1, which the exact remainder decides.  A root of a
+// 53-bit significand is never halfway between two 53-bit numbers either.
+SW_HD double sqrt_int_from(double x, uint32_t &bad, float y) {
+    const uint32_t xh = f64_hi(x), xl = f64_lo(x), ex = xh >> 20, odd = ex & 1u;  // odd: x's exponent is even
+    const uint64_t n = ((uint64_t)(shl_hi(xl, xh, 11) | 0x80000000u) << 32) | (xl << 11);
+    const uint64_t M = n >> odd;
+    const uint32_t y23 = frac23(y) - 4u, y32 = y23 << 9;
+    const uint32_t s0 = mulhi((uint32_t)(M >> 32), y32) << 1;
+    const uint64_t r0 = M - wide(s0, s0);
+    const uint32_t s1 = s0 + (mulhi((uint32_t)(r0 >> 14), y32) >> 18) - 1u;
+    const uint64_t r1 = M - wide(s1, s1);
+    const uint32_t Y = rcp_newton(s1 > 0x80000000u ? s1 : 0x80000000u, y23);
+    const uint32_t d = (mulhi((uint32_t)(r1 >> 3), Y) - 4u) >> 6;
+    // M 2^46 - (s1 2^23 + d)^2
+    const uint64_t t = (r1 << 23) - (wide(s1, d) << 1);
+    const uint64_t rem = (t << 23) - wide(d, d);
+    const uint64_t S = wide(s1, 1u << 23) + d;
+    const uint64_t m = (S + 2u + (uint32_t)(rem > (S << 1))) >> 2;
+    bad |= (uint32_t)!(ex - 1u < 2046u);  // positive and normal
+    const uint32_t e = (((ex + 1023u) >> 1) - 1u) << 20;
+    return f64_of(e + (uint32_t)(m >> 32), (uint32_t)m);
+}
+SW_HD float sqrt_int_arg(double x) {  // x's significand in [1, 4), 24 bits
+    const uint32_t xh = f64_hi(x), xl = f64_lo(x);
+    return f32_from_bits((0x40000000u - (((xh >> 20) & 1u) << 23)) | (shl_hi(xl, xh, 3) & 0x007fffffu));
+}
+SW_HD double sqrt_int_fast(double x, uint32_t &bad) { return sqrt_int_from(x, bad, f32_rsqrt_seed(sqrt_int_arg(x))); }
 
 SW_HD double mul_int(double x, double y) {
     uint32_t bad = 0;

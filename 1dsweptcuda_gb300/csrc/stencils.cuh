@@ -68,6 +68,16 @@ SW_HD float mlp2(float x, float f, int) { return ml(x, f); }
 // the value must be recomputed with ml.  FP32 multiplies.
 SW_HD double mlq(double a, double b, uint32_t &bad) { return mul_int_fast(a, b, bad); }
 SW_HD float mlq(float a, float b, uint32_t &) { return ml(a, b); }
+// Quotients and square roots on the integer pipe, flagged the same way; rcq
+// holds a divisor's reciprocal for the quotients that share it.  FP32 divides.
+SW_HD RcpInt rcq(double b) { return rcp_int(b); }
+SW_HD float rcq(float b) { return b; }
+SW_HD double dvq(double a, const RcpInt &b, uint32_t &bad) { return div_int_with(a, b, bad); }
+SW_HD float dvq(float a, float b, uint32_t &) { return dv(a, b); }
+SW_HD double sqq(double a, uint32_t &bad) { return sqrt_int_fast(a, bad); }
+SW_HD float sqq(float a, uint32_t &) { return sq(a); }
+SW_HD double mlp2q(double x, double, int k, uint32_t &bad) { return mul_pow2_fast(x, k, bad); }
+SW_HD float mlp2q(float x, float f, int, uint32_t &) { return ml(x, f); }
 
 // ---------------------------------------------------------------- Heat
 // execFunc, Heat1D_SweptShared.cu:121-130: fourier*(T[l] + T[r]) + fourierTwo*T[c]
@@ -275,6 +285,54 @@ SW_HD void eu_iface(const Params<T> &p, Q3<T> am, Q3<T> a, Q3<T> b, Q3<T> bp, T 
     const Q3<T> tR = skipB ? b : eu_limit(b, a, dv(ml(bp.x, Db), ml(a.x, Dbp)));
     F = eu_flux(p, tL, tR);
     S = eu_spectral(p, tL, tR);
+}
+// Zero and sign tests without FP64 comparisons, which hold the FP64 pipe like
+// any other FP64 instruction.  same_sign: both below zero or neither, for
+// numbers other than zeros and NaNs (eu_iface_q flags those operands).
+SW_HD bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
+SW_HD bool is_zero(float x) { return x == 0.0f; }
+SW_HD bool same_sign(double a, double b) { return (int32_t)(f64_hi(a) ^ f64_hi(b)) >= 0; }
+SW_HD bool same_sign(float a, float b) { return (a < 0.0f) == (b < 0.0f); }
+SW_HD bool not_finite(double x) { return (f64_hi(x) & 0x7ff00000u) == 0x7ff00000u; }
+SW_HD bool not_finite(float) { return false; }
+// min(r, 1) / 2 of a ratio that dvq did not flag
+SW_HD double half_min1(double r, uint32_t &bad) {
+    return mul_pow2_fast((int32_t)f64_hi(r) >= 0x3ff00000 ? 1.0 : r, -1, bad);
+}
+SW_HD float half_min1(float r, uint32_t &) { return ml(mn(r, 1.0f), 0.5f); }
+// eu_iface with its quotients (seven), square roots (three), halvings and
+// comparisons on the integer pipe (exact_int.h), the same values bit for bit:
+// in FP64 a correctly rounded quotient or root takes eight or more FP64-pipe
+// instructions in software, about half of what an interface issues.  bad is
+// set where an operand is outside that arithmetic's range; F and S are then
+// meaningless and the caller forms them with eu_iface.
+template <typename T>
+SW_HD void eu_iface_q(const Params<T> &p, Q3<T> am, Q3<T> a, Q3<T> b, Q3<T> bp, T Da, T Db, T Dbp, Q3<T> &F, Q3<T> &S,
+                      uint32_t &bad) {
+    bad |= (uint32_t)(not_finite(Da) || not_finite(Db) || not_finite(Dbp));
+    const bool zb = is_zero(Db);
+    Q3<T> L = a, R = b;
+    if (!(is_zero(Da) || zb || !same_sign(Da, Db)))
+        L = qadd(a, qscale(half_min1(dvq(ml(am.x, Db), rcq(ml(b.x, Da)), bad), bad), qsub(b, a)));
+    if (!(zb || is_zero(Dbp) || !same_sign(Db, Dbp)))
+        R = qadd(b, qscale(half_min1(dvq(ml(bp.x, Db), rcq(ml(a.x, Dbp)), bad), bad), qsub(a, b)));
+    // eu_flux
+    const auto iL = rcq(L.x), iR = rcq(R.x);
+    const T uL = dvq(L.y, iL, bad), uR = dvq(R.y, iR, bad);
+    const T pL = ml(p.mgam, sb(L.z, dvq(ml(mlp2q(L.y, T(0.5), -1, bad), L.y), iL, bad)));
+    const T pR = ml(p.mgam, sb(R.z, dvq(ml(mlp2q(R.y, T(0.5), -1, bad), R.y), iR, bad)));
+    F.x = ad(L.y, R.y);
+    F.y = ad(ad(ad(ml(L.y, uL), ml(R.y, uR)), pL), pR);
+    F.z = ad(ad(ad(ml(L.z, uL), ml(R.z, uR)), ml(uL, pL)), ml(uR, pR));
+    // eu_spectral
+    const T rl = sqq(L.x, bad), rr = sqq(R.x, bad);
+    Q3<T> h;
+    h.x = ml(rl, rr);
+    const T hd = dvq(T(1), rcq(ml(h.x, ad(rl, rr))), bad);
+    h.y = ml(ad(ml(rl, R.y), ml(rr, L.y)), hd);
+    h.z = ml(ad(ml(rl, R.z), ml(rr, L.z)), hd);
+    const T pH = ml(p.mgam, sb(h.z, ml(mlp2q(h.y, T(0.5), -1, bad), h.y)));
+    S = qscale(ad(sqq(ml(pH, p.gam), bad), ab(h.y)), qsub(L, R));
 }
 template <typename T>
 SW_HD Q3<T> eu_combine(Q3<T> Fl, Q3<T> Sl, Q3<T> Fr, Q3<T> Sr) {
