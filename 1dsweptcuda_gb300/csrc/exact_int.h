@@ -71,16 +71,6 @@ SW_HD double mul_pow2(double x, double f, int k) {
     return f64_mul_pipe(x, f);
 }
 
-// The same with a flag instead of the fallback (see mul_int_fast below); a
-// zero is its own product.
-SW_HD double mul_pow2_fast(double x, int k, uint32_t &bad) {
-    const uint64_t b = f64_bits(x);
-    const uint32_t e = (uint32_t)(b >> 52) & 0x7ffu;
-    const bool zero = (b << 1) == 0;
-    bad |= (uint32_t)!(zero || (e - 1u < 2046u && e + (uint32_t)k - 1u < 2046u));
-    return f64_from_bits(zero ? b : b + ((uint64_t)(int64_t)k << 52));
-}
-
 // x * 6.
 SW_HD double mul6(double x) {
     const uint64_t b = f64_bits(x);
@@ -115,7 +105,8 @@ SW_HD double mul6(double x) {
 // No FP64 instruction sits on their path, so none is issued: a predicated-off
 // FP64 instruction still holds the FP64 pipe, and a fallback inside the
 // product measured as slow as the multiply it replaces.
-// mul_int, div_int and sqrt_int hold that fallback (host checks).
+// mul_int holds that fallback (host checks); mul_any, div_any and sqrt_any
+// call it.
 SW_HD uint32_t f64_hi(double x) {
 #if defined(__CUDA_ARCH__)
     return (uint32_t)__double2hiint(x);
@@ -343,6 +334,88 @@ SW_HD double mul_int(double x, double y) {
     uint32_t bad = 0;
     const double r = mul_int_fast(x, y, bad);
     return bad ? f64_mul_pipe(x, y) : r;
+}
+
+// ---- the same with the fallback at each operation, for Euler's long chains
+//
+// A cell-level flag and a second evaluation suit Heat and KS, whose cells leave
+// the range together and rarely.  In an Euler run they do not: ahead of every
+// front lies a band of cells whose momenta fall from 1e-16 to nothing, and each
+// of them underflows in a product or two.  So each operation that meets such an
+// operand calls the FP64 instruction itself.  The call keeps it out of line: a
+// fallback that the compiler can turn into a predicated FP64 instruction costs
+// as much as the FP64 operation would (8192 cells, tile 128: 11.0 ms for 256
+// steps with one flag per interface, 8.9 ms on the FP64 pipe alone).
+#if defined(__CUDACC__)
+#define SW_SLOW static __host__ __device__ __noinline__
+#else
+#define SW_SLOW static
+#endif
+SW_SLOW double slow_mul(double x, double y) {
+#if defined(__CUDA_ARCH__)
+    return __dmul_rn(x, y);
+#else
+    return x * y;
+#endif
+}
+SW_SLOW double slow_div(double x, double y) {
+#if defined(__CUDA_ARCH__)
+    return __ddiv_rn(x, y);
+#else
+    return x / y;
+#endif
+}
+SW_SLOW double slow_sqrt(double x) {
+#if defined(__CUDA_ARCH__)
+    return __dsqrt_rn(x);
+#else
+    return __builtin_sqrt(x);
+#endif
+}
+SW_SLOW double slow_half_min1(double r) {
+    const double m = __builtin_fmin(r, 1.0);
+#if defined(__CUDA_ARCH__)
+    return __dmul_rn(0.5, m);
+#else
+    return 0.5 * m;
+#endif
+}
+SW_HD double mul_any(double x, double y) {
+    uint32_t bad = 0;
+    double r = mul_int_fast(x, y, bad);
+    if (bad) r = slow_mul(x, y);
+    return r;
+}
+SW_HD double div_any(double a, double b, const RcpInt &ib) {
+    uint32_t bad = 0;
+    double r = div_int_with(a, ib, bad);
+    if (bad) r = slow_div(a, b);
+    return r;
+}
+SW_HD double sqrt_any(double x) {
+    uint32_t bad = 0;
+    double r = sqrt_int_fast(x, bad);
+    if (bad) r = slow_sqrt(x);
+    return r;
+}
+// x 2^k, k = -1 or 1 (f = 2^k)
+SW_HD double pow2_any(double x, double f, int k) {
+    const uint32_t hi = f64_hi(x);
+    if (((hi >> 20) & 0x7ffu) - 2u < 2043u) return f64_of(hi + ((uint32_t)k << 20), f64_lo(x));
+    return slow_mul(x, f);
+}
+// 0.5 min(r, 1), a NaN counting as 1 (fmin)
+SW_HD double half_min1_any(double r) {
+    const uint32_t hi = f64_hi(r);
+    if ((int32_t)hi >= 0x3ff00000) return 0.5;  // 1 and above, infinity, NaN
+    if (((hi >> 20) & 0x7ffu) - 2u < 2043u) return f64_of(hi - (1u << 20), f64_lo(r));
+    return slow_half_min1(r);
+}
+// x == 0 and x < 0 without an FP64 comparison (which holds the FP64 pipe too)
+SW_HD bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
+SW_HD bool is_neg(double x) {
+    const uint64_t b = f64_bits(x);
+    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
 }
 
 }  // namespace sw

@@ -134,8 +134,13 @@ __device__ __forceinline__ bool persistent_tile(const Params<T> &p, typename Sch
     return true;
 }
 
+// FP64 Euler: as many blocks per SM as its launch-per-pass kernels.
+template <int P, typename T>
+constexpr int persistent_min_blocks() {
+    return P == SW_EULER && sizeof(T) == 8 ? SW_EULER_MIN_BLOCKS : 0;
+}
 template <int P, typename T, int PATH>
-__global__ void __launch_bounds__(Scheme<P, T>::MAXT)
+__global__ void __launch_bounds__(Scheme<P, T>::MAXT, (persistent_min_blocks<P, T>()))
     k_persistent(const Params<T> p, typename Scheme<P, T>::G *__restrict__ state,
                  typename Scheme<P, T>::G *__restrict__ slots, unsigned *__restrict__ flags, int *status, const int W,
                  const int64_t n_diamonds) {
@@ -342,7 +347,7 @@ __global__ void __launch_bounds__(kClassicBlock)
 }
 
 template <int P, typename T, int PATH>
-__global__ void __launch_bounds__(Scheme<P, T>::MAXT)
+__global__ void __launch_bounds__(Scheme<P, T>::MAXT, (persistent_min_blocks<P, T>()))
     k_persistent_batch(const Params<T> p, typename Scheme<P, T>::G *__restrict__ state,
                        typename Scheme<P, T>::G *__restrict__ slots, const BatchDev b, unsigned *__restrict__ flags,
                        int *status, const int W, const int64_t n_diamonds) {

@@ -68,16 +68,35 @@ SW_HD float mlp2(float x, float f, int) { return ml(x, f); }
 // the value must be recomputed with ml.  FP32 multiplies.
 SW_HD double mlq(double a, double b, uint32_t &bad) { return mul_int_fast(a, b, bad); }
 SW_HD float mlq(float a, float b, uint32_t &) { return ml(a, b); }
-// Quotients and square roots on the integer pipe, flagged the same way; rcq
-// holds a divisor's reciprocal for the quotients that share it.  FP32 divides.
-SW_HD RcpInt rcq(double b) { return rcp_int(b); }
+// Euler's operations: on the integer pipe in FP64 (exact_int.h), the FP64
+// instruction wherever an operand is outside its range; plain in FP32.  rcq
+// holds a divisor and its reciprocal for the quotients that share it.
+struct Divisor {
+    double d;
+    RcpInt i;
+};
+SW_HD Divisor rcq(double b) { return Divisor{b, rcp_int(b)}; }
 SW_HD float rcq(float b) { return b; }
-SW_HD double dvq(double a, const RcpInt &b, uint32_t &bad) { return div_int_with(a, b, bad); }
-SW_HD float dvq(float a, float b, uint32_t &) { return dv(a, b); }
-SW_HD double sqq(double a, uint32_t &bad) { return sqrt_int_fast(a, bad); }
-SW_HD float sqq(float a, uint32_t &) { return sq(a); }
-SW_HD double mlp2q(double x, double, int k, uint32_t &bad) { return mul_pow2_fast(x, k, bad); }
-SW_HD float mlp2q(float x, float f, int, uint32_t &) { return ml(x, f); }
+SW_HD double dvq(double a, const Divisor &b) { return div_any(a, b.d, b.i); }
+SW_HD float dvq(float a, float b) { return dv(a, b); }
+SW_HD double sqq(double a) { return sqrt_any(a); }
+SW_HD float sqq(float a) { return sq(a); }
+SW_HD double half(double x) { return pow2_any(x, 0.5, -1); }
+SW_HD float half(float x) { return ml(0.5f, x); }
+SW_HD double twice(double x) { return pow2_any(x, 2.0, 1); }
+SW_HD float twice(float x) { return ml(2.0f, x); }
+SW_HD double half_min1(double r) { return half_min1_any(r); }
+SW_HD float half_min1(float r) { return ml(mn(r, 1.0f), 0.5f); }
+SW_HD bool is_zero(float x) { return x == 0.0f; }
+SW_HD bool is_neg(float x) { return x < 0.0f; }
+// b - a from d = a - b: -d, but equal values differ by +0 both ways
+SW_HD double neg_diff(double d) { return f64_from_bits(f64_bits(d) == 0 ? 0 : f64_bits(d) ^ 0x8000000000000000ull); }
+SW_HD float neg_diff(float d) { return d == 0.0f ? 0.0f : -d; }
+// a product on the integer pipe (INT) or the FP64 pipe
+template <bool INT>
+SW_HD double mle(double a, double b) { return INT ? mul_any(a, b) : ml(a, b); }
+template <bool INT>
+SW_HD float mle(float a, float b) { return ml(a, b); }
 
 // ---------------------------------------------------------------- Heat
 // execFunc, Heat1D_SweptShared.cu:121-130: fourier*(T[l] + T[r]) + fourierTwo*T[c]
@@ -286,57 +305,67 @@ SW_HD void eu_iface(const Params<T> &p, Q3<T> am, Q3<T> a, Q3<T> b, Q3<T> bp, T 
     F = eu_flux(p, tL, tR);
     S = eu_spectral(p, tL, tR);
 }
-// Zero and sign tests without FP64 comparisons, which hold the FP64 pipe like
-// any other FP64 instruction.  same_sign: both below zero or neither, for
-// numbers other than zeros and NaNs (eu_iface_q flags those operands).
-SW_HD bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
-SW_HD bool is_zero(float x) { return x == 0.0f; }
-SW_HD bool same_sign(double a, double b) { return (int32_t)(f64_hi(a) ^ f64_hi(b)) >= 0; }
-SW_HD bool same_sign(float a, float b) { return (a < 0.0f) == (b < 0.0f); }
-SW_HD bool not_finite(double x) { return (f64_hi(x) & 0x7ff00000u) == 0x7ff00000u; }
-SW_HD bool not_finite(float) { return false; }
-// min(r, 1) / 2 of a ratio that dvq did not flag
-SW_HD double half_min1(double r, uint32_t &bad) {
-    return mul_pow2_fast((int32_t)f64_hi(r) >= 0x3ff00000 ? 1.0 : r, -1, bad);
-}
-SW_HD float half_min1(float r, uint32_t &) { return ml(mn(r, 1.0f), 0.5f); }
-// eu_iface with its quotients (seven), square roots (three), halvings and
-// comparisons on the integer pipe (exact_int.h), the same values bit for bit:
-// in FP64 a correctly rounded quotient or root takes eight or more FP64-pipe
-// instructions in software, about half of what an interface issues.  bad is
-// set where an operand is outside that arithmetic's range; F and S are then
-// meaningless and the caller forms them with eu_iface.
+// eu_pdiff with its products on the integer pipe.
 template <typename T>
-SW_HD void eu_iface_q(const Params<T> &p, Q3<T> am, Q3<T> a, Q3<T> b, Q3<T> bp, T Da, T Db, T Dbp, Q3<T> &F, Q3<T> &S,
-                      uint32_t &bad) {
-    bad |= (uint32_t)(not_finite(Da) || not_finite(Db) || not_finite(Dbp));
-    const bool zb = is_zero(Db);
+SW_HD T eu_pdiff_q(Q3<T> a, Q3<T> b) {
+    return ad(mle<true>(mle<true>(twice(b.x), a.x), sb(b.z, a.z)),
+              sb(mle<true>(mle<true>(a.y, a.y), b.x), mle<true>(mle<true>(b.y, b.y), a.x)));
+}
+template <bool INT, typename T>
+SW_HD Q3<T> qscale_q(T s, Q3<T> a) {
+    return q3(mle<INT>(s, a.x), mle<INT>(s, a.y), mle<INT>(s, a.z));
+}
+// eu_iface with its quotients (seven), square roots (three), halvings,
+// comparisons and products on the integer pipe (exact_int.h), the same values
+// bit for bit: of about 190 FP64 instructions per interface and cell in
+// software (a correctly rounded quotient or root takes eight or more), the sums
+// remain.  b - a serves both limited states, a - b being its negative.
+// LIM: the limiter's products too.  At 2^21 cells, FP64, cell-updates/s:
+// classic 1.41e9 all on the FP64 pipe, 2.77e9 with the quotients and roots
+// moved, 3.90e9 with every product (eu_pdiff_q and eu_advance_q included).  A
+// swept level ends in barriers, which the longer integer chains reach later:
+// 1.48e9, 2.80e9, then 3.31e9 with the flux and spectral products, 3.28e9 with
+// the limiter's as well and 3.20e9 with every product.  So classic sets LIM and
+// the swept levels do not.
+template <bool LIM, typename T>
+SW_HD void eu_iface_q(const Params<T> &p, Q3<T> am, Q3<T> a, Q3<T> b, Q3<T> bp, T Da, T Db, T Dbp, Q3<T> &F, Q3<T> &S) {
+    const bool zb = is_zero(Db), nb = is_neg(Db);
+    const bool limL = !(is_zero(Da) || zb || is_neg(Da) != nb), limR = !(zb || is_zero(Dbp) || is_neg(Dbp) != nb);
     Q3<T> L = a, R = b;
-    if (!(is_zero(Da) || zb || !same_sign(Da, Db)))
-        L = qadd(a, qscale(half_min1(dvq(ml(am.x, Db), rcq(ml(b.x, Da)), bad), bad), qsub(b, a)));
-    if (!(zb || is_zero(Dbp) || !same_sign(Db, Dbp)))
-        R = qadd(b, qscale(half_min1(dvq(ml(bp.x, Db), rcq(ml(a.x, Dbp)), bad), bad), qsub(a, b)));
+    if (limL || limR) {
+        const Q3<T> d = qsub(b, a);
+        if (limL) L = qadd(a, qscale_q<LIM>(half_min1(dvq(mle<LIM>(am.x, Db), rcq(mle<LIM>(b.x, Da)))), d));
+        if (limR)
+            R = qadd(b, qscale_q<LIM>(half_min1(dvq(mle<LIM>(bp.x, Db), rcq(mle<LIM>(a.x, Dbp)))),
+                                      q3(neg_diff(d.x), neg_diff(d.y), neg_diff(d.z))));
+    }
     // eu_flux
     const auto iL = rcq(L.x), iR = rcq(R.x);
-    const T uL = dvq(L.y, iL, bad), uR = dvq(R.y, iR, bad);
-    const T pL = ml(p.mgam, sb(L.z, dvq(ml(mlp2q(L.y, T(0.5), -1, bad), L.y), iL, bad)));
-    const T pR = ml(p.mgam, sb(R.z, dvq(ml(mlp2q(R.y, T(0.5), -1, bad), R.y), iR, bad)));
+    const T uL = dvq(L.y, iL), uR = dvq(R.y, iR);
+    const T pL = mle<true>(p.mgam, sb(L.z, dvq(mle<true>(half(L.y), L.y), iL)));
+    const T pR = mle<true>(p.mgam, sb(R.z, dvq(mle<true>(half(R.y), R.y), iR)));
     F.x = ad(L.y, R.y);
-    F.y = ad(ad(ad(ml(L.y, uL), ml(R.y, uR)), pL), pR);
-    F.z = ad(ad(ad(ml(L.z, uL), ml(R.z, uR)), ml(uL, pL)), ml(uR, pR));
+    F.y = ad(ad(ad(mle<true>(L.y, uL), mle<true>(R.y, uR)), pL), pR);
+    F.z = ad(ad(ad(mle<true>(L.z, uL), mle<true>(R.z, uR)), mle<true>(uL, pL)), mle<true>(uR, pR));
     // eu_spectral
-    const T rl = sqq(L.x, bad), rr = sqq(R.x, bad);
+    const T rl = sqq(L.x), rr = sqq(R.x);
     Q3<T> h;
-    h.x = ml(rl, rr);
-    const T hd = dvq(T(1), rcq(ml(h.x, ad(rl, rr))), bad);
-    h.y = ml(ad(ml(rl, R.y), ml(rr, L.y)), hd);
-    h.z = ml(ad(ml(rl, R.z), ml(rr, L.z)), hd);
-    const T pH = ml(p.mgam, sb(h.z, ml(mlp2q(h.y, T(0.5), -1, bad), h.y)));
-    S = qscale(ad(sqq(ml(pH, p.gam), bad), ab(h.y)), qsub(L, R));
+    h.x = mle<true>(rl, rr);
+    const T hd = dvq(T(1), rcq(mle<true>(h.x, ad(rl, rr))));
+    h.y = mle<true>(ad(mle<true>(rl, R.y), mle<true>(rr, L.y)), hd);
+    h.z = mle<true>(ad(mle<true>(rl, R.z), mle<true>(rr, L.z)), hd);
+    const T pH = mle<true>(p.mgam, sb(h.z, mle<true>(half(h.y), h.y)));
+    S = qscale_q<true>(ad(sqq(mle<true>(pH, p.gam)), ab(h.y)), qsub(L, R));
 }
 template <typename T>
 SW_HD Q3<T> eu_combine(Q3<T> Fl, Q3<T> Sl, Q3<T> Fr, Q3<T> Sr) {
     return qsub(qsub(qadd(Fl, Sl), Fr), Sr);
+}
+
+// A cell's new value u + scale * sum, the product on the integer pipe.
+template <typename T>
+SW_HD Q3<T> eu_advance_q(Q3<T> u, T scale, Q3<T> sum) {
+    return qadd(u, qscale_q<true>(scale, sum));
 }
 
 // eulerStutterStep result, :345: s2 + (0.25*dt_dx)*flux
