@@ -96,7 +96,9 @@ int ensure_tables(sw_ctx *ctx, int32_t n, const int64_t *nx, int W) {
     int32_t group = 4;  // grouped swept blocks (G tiles of one domain each) where every domain allows them
     for (int32_t d = 0; d < n && W; ++d)
         while (group > 1 && (nx[d] / W) % group != 0) group >>= 1;
-    bt.dev = BatchDev{d_dom, d_off, d_tile0, d_blk, tiles, cells, n, W ? group : 1};
+    int32_t vec4 = 1;
+    for (int32_t d = 0; d < n; ++d) vec4 = vec4 && nx[d] % 4 == 0;
+    bt.dev = BatchDev{d_dom, d_off, d_tile0, d_blk, tiles, cells, n, W ? group : 1, vec4};
     bt.nx.assign(nx, nx + n);
     bt.W = W;
     if (ctx->graph.exec) {  // the tables moved: a cached graph may point at the old ones

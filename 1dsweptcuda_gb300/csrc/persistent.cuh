@@ -337,6 +337,7 @@ __global__ void __launch_bounds__(kClassicBlock)
     k_classic_batch(const Params<T> p, const typename Scheme<P, T>::G *__restrict__ in,
                     typename Scheme<P, T>::G *__restrict__ out, const BatchDev b, const int sub) {
     const int64_t g = (int64_t)blockIdx.x * kClassicBlock + threadIdx.x;
+    wait_for_previous_launch();
     if (g >= b.n_cells) return;
     int d = b.blk_dom[blockIdx.x];
     while (b.off[d + 1] <= g) ++d;
@@ -344,6 +345,23 @@ __global__ void __launch_bounds__(kClassicBlock)
     Params<T> q = p;
     q.nx = b.off[d + 1] - off;
     classic_cell<P, T>(q, in + off, out + off, sub, g - off);
+}
+
+// FP32 Heat / KS, four cells per thread (classic_cells4); every domain length a
+// multiple of 4 (BatchDev::vec4).
+template <int P>
+__global__ void __launch_bounds__(kClassicBlock)
+    k_classic4_batch(const Params<float> p, const float *__restrict__ in, float *__restrict__ out, const BatchDev b,
+                     const int sub) {
+    const int64_t g = 4 * ((int64_t)blockIdx.x * kClassicBlock + threadIdx.x);
+    wait_for_previous_launch();
+    if (g >= b.n_cells) return;
+    int d = b.blk_dom[g / kClassicBlock];
+    while (b.off[d + 1] <= g) ++d;
+    const int64_t off = b.off[d];
+    Params<float> q = p;
+    q.nx = b.off[d + 1] - off;
+    classic_cells4<P>(q, in + off, out + off, sub, g - off);
 }
 
 template <int P, typename T, int PATH>
@@ -499,10 +517,15 @@ cudaError_t launch_classic_batch(const void *vp, const void *in, void *out, int 
     const Params<T> &p = *static_cast<const Params<T> *>(vp);
     const BatchDev &b = *static_cast<const BatchDev *>(bt);
     (void)block;  // the block is fixed by the domain table's granularity
+    const G *gin = static_cast<const G *>(in);
+    G *gout = static_cast<G *>(out);
+    if constexpr (P != SW_EULER && sizeof(T) == 4) {
+        if (b.vec4 && aligned16(in, out))
+            return launch_dependent(k_classic4_batch<P>, (unsigned)((b.n_cells / 4 + kClassicBlock - 1) / kClassicBlock),
+                                    kClassicBlock, s, p, gin, gout, b, sub);
+    }
     const int64_t grid = (b.n_cells + kClassicBlock - 1) / kClassicBlock;
-    k_classic_batch<P, T><<<(unsigned)grid, kClassicBlock, 0, s>>>(p, static_cast<const G *>(in), static_cast<G *>(out),
-                                                                    b, sub);
-    return cudaGetLastError();
+    return launch_dependent(k_classic_batch<P, T>, (unsigned)grid, kClassicBlock, s, p, gin, gout, b, sub);
 }
 
 // Cooperative launch through cudaLaunchKernelEx so that it can be captured

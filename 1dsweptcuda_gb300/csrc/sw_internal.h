@@ -43,6 +43,7 @@ struct BatchDev {
     int64_t n_cells;
     int32_t n_dom;
     int32_t group;  // the largest of 1, 2, 4 that divides every domain's tile count
+    int32_t vec4;   // every domain length is a multiple of 4
 };
 constexpr int kClassicBlock = 256;  // threads (= cells) per block of the ensemble classic kernel
 
