@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "ctx.h"
+#include "launch.cuh"
 #include "stencils.cuh"
 #include "sw_internal.h"
 
@@ -333,6 +334,7 @@ __global__ void __launch_bounds__(THREADS) k_step(const float *__restrict__ thet
     extern __shared__ __align__(16) unsigned char raw[];
     Smem &s = *reinterpret_cast<Smem *>(raw);
     const int64_t dom = blockIdx.x / tiles_per_dom, x0 = (blockIdx.x % tiles_per_dom) * TOUT;
+    wait_for_previous_launch();
     load_tile(s, theta, u + dom * n, n, x0, w2p, use_closure != 0);  // theta may be null without the closure
     __syncthreads();
     if (use_closure) forward_12<false>(s);
@@ -680,8 +682,8 @@ int closure_enqueue(sw_ctx *ctx, const sw_config *coarse, const float *theta, fl
         if (rc) return rc;
     }
     for (int64_t i = 0; i < n_steps; ++i) {
-        cl::k_step<<<(unsigned)(tiles * n_dom), cl::THREADS, cl::smem_fwd_bytes(), ctx->stream>>>(
-            theta, w2p, p, cur, alt, n, tiles, use_closure);
+        SW_CUDA(ctx, launch_dependent(cl::k_step, (unsigned)(tiles * n_dom), cl::THREADS, cl::smem_fwd_bytes(), ctx->stream,
+                                      theta, w2p, p, cur, alt, n, tiles, use_closure));
         std::swap(cur, alt);
     }
     SW_CUDA(ctx, cudaGetLastError());

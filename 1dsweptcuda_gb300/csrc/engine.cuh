@@ -33,6 +33,7 @@
 #include <cstdint>
 #include <type_traits>
 
+#include "launch.cuh"
 #include "stencils.cuh"
 #include "sw_internal.h"
 
@@ -735,6 +736,7 @@ __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PA
                                                 typename Scheme<P, T>::G *__restrict__ slots, const int W,
                                                 const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     swept_tile<P, T, MODE, PATH>(p, state, slots, reinterpret_cast<T *>(sw_smem), W, phase, (int64_t)blockIdx.x);
 }
 
@@ -825,16 +827,6 @@ __device__ __forceinline__ void classic_cell(const Params<T> &p, const typename 
         out[g] = V4<T>{o.x, o.y, o.z, T(0)};
     }
 }
-
-// A classic step is a chain of short launches, and a launch that starts when the
-// one before it has drained costs 4 us whatever it does.  launch_dependent lets a
-// launch be scheduled earlier (programmatic dependent launch); it waits here,
-// before its first access, for the previous one to have completed and its
-// writes to be visible: 1.6 us per launch on small domains.  The previous
-// kernel's blocks release it as they exit, not before: released at their start,
-// its blocks settled on SMs still at work and left others idle (KS FP64, 65536
-// cells: 4.9 ms for 600 launches, 1.8 as it is, 3.6 without any of this).
-__device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // FP32 Heat / KS with four consecutive cells per thread and 16-byte accesses (in
 // and out 16-byte aligned, nx a multiple of 4).  One cell per thread left the
@@ -1147,6 +1139,7 @@ template <int P, typename T, int MODE, int G, int PATH>
 __global__ void __launch_bounds__(1024, 2) k_swept_group(const Params<T> p, T *__restrict__ state,
                                                       T *__restrict__ slots, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     swept_tile_group<P, T, MODE, G, PATH>(p, state, slots, reinterpret_cast<T *>(sw_smem), W, phase,
                                           G * (int64_t)blockIdx.x);
 }
@@ -1177,21 +1170,6 @@ struct SmemOnce {
     }
 };
 
-// A launch that may be scheduled while the launch before it drains
-// (wait_for_previous_launch).
-template <typename... K, typename... A>
-cudaError_t launch_dependent(void (*kernel)(K...), unsigned grid, unsigned block, cudaStream_t s, A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
-}
 inline bool aligned16(const void *a, const void *b) { return (((uintptr_t)a | (uintptr_t)b) & 15) == 0; }
 
 template <int P, typename T>
@@ -1203,15 +1181,15 @@ cudaError_t launch_classic(const void *vp, const void *in, void *out, int sub, i
     G *gout = static_cast<G *>(out);
     if constexpr (P == SW_EULER) {
         const int64_t warps = (nx + kEulerCellsPerWarp - 1) / kEulerCellsPerWarp;
-        return launch_dependent(k_classic_euler<T>, (unsigned)((warps + 7) / 8), 256, s, p, gin, gout, sub);
+        return launch_dependent(k_classic_euler<T>, (unsigned)((warps + 7) / 8), 256, 0, s, p, gin, gout, sub);
     }
     if constexpr (P != SW_EULER && sizeof(T) == 4) {
         if (aligned16(in, out) && nx % 4 == 0)
-            return launch_dependent(k_classic4<P>, (unsigned)((nx / 4 + 255) / 256), 256, s, p, gin, gout, sub);
+            return launch_dependent(k_classic4<P>, (unsigned)((nx / 4 + 255) / 256), 256, 0, s, p, gin, gout, sub);
     }
     if (block <= 0 || block > Scheme<P, T>::CMAXT) block = block <= 0 ? 256 : Scheme<P, T>::CMAXT;
     const int64_t grid = (nx + block - 1) / block;
-    return launch_dependent(k_classic<P, T>, (unsigned)grid, block, s, p, gin, gout, sub);
+    return launch_dependent(k_classic<P, T>, (unsigned)grid, block, 0, s, p, gin, gout, sub);
 }
 
 template <int P, typename T, int PATH>
@@ -1224,11 +1202,10 @@ cudaError_t launch_swept_path(const Params<T> &p, int mode, int phase, typename 
     const size_t smem = swept_smem_bytes<P, T>(W);
     const unsigned grid = (unsigned)(nx / W);
     switch (mode) {
-    case MODE_UP: k_swept<P, T, MODE_UP, PATH><<<grid, threads, smem, s>>>(p, st, sl, W, phase); break;
-    case MODE_DIAMOND: k_swept<P, T, MODE_DIAMOND, PATH><<<grid, threads, smem, s>>>(p, st, sl, W, phase); break;
-    default: k_swept<P, T, MODE_DOWN, PATH><<<grid, threads, smem, s>>>(p, st, sl, W, phase); break;
+    case MODE_UP: return launch_dependent(k_swept<P, T, MODE_UP, PATH>, grid, threads, smem, s, p, st, sl, W, phase);
+    case MODE_DIAMOND: return launch_dependent(k_swept<P, T, MODE_DIAMOND, PATH>, grid, threads, smem, s, p, st, sl, W, phase);
+    default: return launch_dependent(k_swept<P, T, MODE_DOWN, PATH>, grid, threads, smem, s, p, st, sl, W, phase);
     }
-    return cudaGetLastError();
 }
 
 // ------------------------------------------------ KS 128-cell tiles in one warp
@@ -1283,6 +1260,7 @@ __global__ void __launch_bounds__(32 * kKsWarpTilesPerBlock)
     const int lane = threadIdx.x & 31, c0 = 4 * lane;
     const int64_t nx = p.nx, nhalf = nx / h;  // ntile: the tiles launched (all, or all but the wrapping one)
     const int64_t t = (int64_t)blockIdx.x * kKsWarpTilesPerBlock + (threadIdx.x >> 5);
+    wait_for_previous_launch();
     if (t >= ntile) return;  // whole warps: t is the same for the 32 lanes
     const int64_t base = t * W + (int64_t)phase * h;
     const int64_t hl = (2 * t + phase) % nhalf;
@@ -1345,13 +1323,11 @@ cudaError_t launch_swept_group(const Params<T> &p, int mode, int phase, T *st, T
     const unsigned grid = (unsigned)(nx / W / G);
     const int block = G * threads;
     switch (mode) {
-    case MODE_UP: k_swept_group<P, T, MODE_UP, G, PATH><<<grid, block, smem, s>>>(p, st, sl, W, phase); break;
+    case MODE_UP: return launch_dependent(k_swept_group<P, T, MODE_UP, G, PATH>, grid, block, smem, s, p, st, sl, W, phase);
     case MODE_DIAMOND:
-        k_swept_group<P, T, MODE_DIAMOND, G, PATH><<<grid, block, smem, s>>>(p, st, sl, W, phase);
-        break;
-    default: k_swept_group<P, T, MODE_DOWN, G, PATH><<<grid, block, smem, s>>>(p, st, sl, W, phase); break;
+        return launch_dependent(k_swept_group<P, T, MODE_DIAMOND, G, PATH>, grid, block, smem, s, p, st, sl, W, phase);
+    default: return launch_dependent(k_swept_group<P, T, MODE_DOWN, G, PATH>, grid, block, smem, s, p, st, sl, W, phase);
     }
-    return cudaGetLastError();
 }
 
 template <typename T>
@@ -1360,11 +1336,10 @@ cudaError_t launch_swept_ks_warp(const Params<T> &p, int mode, int phase, T *st,
     const unsigned grid = (unsigned)((ntile + kKsWarpTilesPerBlock - 1) / kKsWarpTilesPerBlock);
     const int threads = 32 * kKsWarpTilesPerBlock;
     switch (mode) {
-    case MODE_UP: k_swept_ks_warp<T, MODE_UP><<<grid, threads, 0, s>>>(p, st, sl, phase, ntile); break;
-    case MODE_DIAMOND: k_swept_ks_warp<T, MODE_DIAMOND><<<grid, threads, 0, s>>>(p, st, sl, phase, ntile); break;
-    default: k_swept_ks_warp<T, MODE_DOWN><<<grid, threads, 0, s>>>(p, st, sl, phase, ntile); break;
+    case MODE_UP: return launch_dependent(k_swept_ks_warp<T, MODE_UP>, grid, threads, 0, s, p, st, sl, phase, ntile);
+    case MODE_DIAMOND: return launch_dependent(k_swept_ks_warp<T, MODE_DIAMOND>, grid, threads, 0, s, p, st, sl, phase, ntile);
+    default: return launch_dependent(k_swept_ks_warp<T, MODE_DOWN>, grid, threads, 0, s, p, st, sl, phase, ntile);
     }
-    return cudaGetLastError();
 }
 
 // A domain of fewer tiles than two per SM of the current device: its levels'

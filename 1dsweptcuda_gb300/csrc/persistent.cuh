@@ -302,6 +302,7 @@ __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PA
     k_swept_batch(const Params<T> p, typename Scheme<P, T>::G *__restrict__ state,
                   typename Scheme<P, T>::G *__restrict__ slots, const BatchDev b, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     const int64_t g = blockIdx.x;
     const int d = b.tile_dom[g];
     const int64_t off = b.off[d];
@@ -319,6 +320,7 @@ __global__ void __launch_bounds__(1024, 2)
     k_swept_batch_group(const Params<T> p, T *__restrict__ state, T *__restrict__ slots, const BatchDev b, const int W,
                         const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     const int64_t g0 = G * (int64_t)blockIdx.x;
     const int d = b.tile_dom[g0];
     const int64_t off = b.off[d];
@@ -449,13 +451,11 @@ cudaError_t launch_swept_batch_path(const Params<T> &p, int mode, int phase, typ
     const size_t smem = swept_smem_bytes<P, T>(W);
     const unsigned grid = (unsigned)b.n_tiles;
     switch (mode) {
-    case MODE_UP: k_swept_batch<P, T, MODE_UP, PATH><<<grid, threads, smem, s>>>(p, st, sl, b, W, phase); break;
+    case MODE_UP: return launch_dependent(k_swept_batch<P, T, MODE_UP, PATH>, grid, threads, smem, s, p, st, sl, b, W, phase);
     case MODE_DIAMOND:
-        k_swept_batch<P, T, MODE_DIAMOND, PATH><<<grid, threads, smem, s>>>(p, st, sl, b, W, phase);
-        break;
-    default: k_swept_batch<P, T, MODE_DOWN, PATH><<<grid, threads, smem, s>>>(p, st, sl, b, W, phase); break;
+        return launch_dependent(k_swept_batch<P, T, MODE_DIAMOND, PATH>, grid, threads, smem, s, p, st, sl, b, W, phase);
+    default: return launch_dependent(k_swept_batch<P, T, MODE_DOWN, PATH>, grid, threads, smem, s, p, st, sl, b, W, phase);
     }
-    return cudaGetLastError();
 }
 
 template <int P, typename T, int G>
@@ -471,14 +471,11 @@ cudaError_t launch_swept_batch_group(const Params<T> &p, int mode, int phase, T 
     const int block = G * W;
     switch (mode) {
     case MODE_UP:
-        k_swept_batch_group<P, T, MODE_UP, G, PATH_CELL><<<grid, block, smem, s>>>(p, st, sl, b, W, phase);
-        break;
+        return launch_dependent(k_swept_batch_group<P, T, MODE_UP, G, PATH_CELL>, grid, block, smem, s, p, st, sl, b, W, phase);
     case MODE_DIAMOND:
-        k_swept_batch_group<P, T, MODE_DIAMOND, G, PATH_CELL><<<grid, block, smem, s>>>(p, st, sl, b, W, phase);
-        break;
-    default: k_swept_batch_group<P, T, MODE_DOWN, G, PATH_CELL><<<grid, block, smem, s>>>(p, st, sl, b, W, phase); break;
+        return launch_dependent(k_swept_batch_group<P, T, MODE_DIAMOND, G, PATH_CELL>, grid, block, smem, s, p, st, sl, b, W, phase);
+    default: return launch_dependent(k_swept_batch_group<P, T, MODE_DOWN, G, PATH_CELL>, grid, block, smem, s, p, st, sl, b, W, phase);
     }
-    return cudaGetLastError();
 }
 
 template <int P, typename T>
@@ -522,10 +519,10 @@ cudaError_t launch_classic_batch(const void *vp, const void *in, void *out, int 
     if constexpr (P != SW_EULER && sizeof(T) == 4) {
         if (b.vec4 && aligned16(in, out))
             return launch_dependent(k_classic4_batch<P>, (unsigned)((b.n_cells / 4 + kClassicBlock - 1) / kClassicBlock),
-                                    kClassicBlock, s, p, gin, gout, b, sub);
+                                    kClassicBlock, 0, s, p, gin, gout, b, sub);
     }
     const int64_t grid = (b.n_cells + kClassicBlock - 1) / kClassicBlock;
-    return launch_dependent(k_classic_batch<P, T>, (unsigned)grid, kClassicBlock, s, p, gin, gout, b, sub);
+    return launch_dependent(k_classic_batch<P, T>, (unsigned)grid, kClassicBlock, 0, s, p, gin, gout, b, sub);
 }
 
 // Cooperative launch through cudaLaunchKernelEx so that it can be captured

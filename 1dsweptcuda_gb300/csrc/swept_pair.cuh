@@ -196,6 +196,7 @@ template <int MODE, int C, bool POW2>
 __global__ void __launch_bounds__(256 / C, (C == 2 ? 8 : 5))
     k_swept_ks_pair(const Params<float> p, float *state, float *slots, const int W, const int phase, const int64_t ntile) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     const int64_t t0 = 2 * (int64_t)blockIdx.x, t1 = t0 + 1 < ntile ? t0 + 1 : t0;
     ks_pair_block<MODE, C, POW2>(p, pair_tile(state, slots, W, phase, t0, p.nx), pair_tile(state, slots, W, phase, t1, p.nx),
                               reinterpret_cast<float2 *>(sw_smem), W);
@@ -206,6 +207,7 @@ template <int MODE, int C, bool POW2>
 __global__ void __launch_bounds__(256 / C, (C == 2 ? 8 : 5))
     k_swept_ks_pair_batch(const Params<float> p, float *state, float *slots, const BatchDev b, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
+    wait_for_previous_launch();
     const int64_t g0 = 2 * (int64_t)blockIdx.x, g1 = g0 + 1 < b.n_tiles ? g0 + 1 : g0;
     auto tile = [&](int64_t g) {
         const int d = b.tile_dom[g];
@@ -237,39 +239,37 @@ inline int pair_chunks(int W, int64_t ntile) {
 }
 
 template <int MODE, int C>
-inline void launch_ks_pair_mode(const Params<float> &p, float *st, float *sl, int W, int phase, int64_t ntile, cudaStream_t s) {
+inline cudaError_t launch_ks_pair_mode(const Params<float> &p, float *st, float *sl, int W, int phase, int64_t ntile, cudaStream_t s) {
     const unsigned grid = (unsigned)((ntile + 1) / 2);
     const size_t smem = pair_smem_bytes(W);
-    if (p.ks_form == KS_POW2) k_swept_ks_pair<MODE, C, true><<<grid, W / 4 / C, smem, s>>>(p, st, sl, W, phase, ntile);
-    else k_swept_ks_pair<MODE, C, false><<<grid, W / 4 / C, smem, s>>>(p, st, sl, W, phase, ntile);
+    if (p.ks_form == KS_POW2) return launch_dependent(k_swept_ks_pair<MODE, C, true>, grid, W / 4 / C, smem, s, p, st, sl, W, phase, ntile);
+    return launch_dependent(k_swept_ks_pair<MODE, C, false>, grid, W / 4 / C, smem, s, p, st, sl, W, phase, ntile);
 }
 template <int C>
 inline cudaError_t launch_ks_pair(const Params<float> &p, int mode, int phase, float *st, float *sl, int64_t nx, int W,
                                   cudaStream_t s) {
     switch (mode) {
-    case MODE_UP: launch_ks_pair_mode<MODE_UP, C>(p, st, sl, W, phase, nx / W, s); break;
-    case MODE_DIAMOND: launch_ks_pair_mode<MODE_DIAMOND, C>(p, st, sl, W, phase, nx / W, s); break;
-    default: launch_ks_pair_mode<MODE_DOWN, C>(p, st, sl, W, phase, nx / W, s); break;
+    case MODE_UP: return launch_ks_pair_mode<MODE_UP, C>(p, st, sl, W, phase, nx / W, s);
+    case MODE_DIAMOND: return launch_ks_pair_mode<MODE_DIAMOND, C>(p, st, sl, W, phase, nx / W, s);
+    default: return launch_ks_pair_mode<MODE_DOWN, C>(p, st, sl, W, phase, nx / W, s);
     }
-    return cudaGetLastError();
 }
 template <int MODE, int C>
-inline void launch_ks_pair_batch_mode(const Params<float> &p, float *st, float *sl, const BatchDev &b, int W, int phase,
+inline cudaError_t launch_ks_pair_batch_mode(const Params<float> &p, float *st, float *sl, const BatchDev &b, int W, int phase,
                                       cudaStream_t s) {
     const unsigned grid = (unsigned)((b.n_tiles + 1) / 2);
     const size_t smem = pair_smem_bytes(W);
-    if (p.ks_form == KS_POW2) k_swept_ks_pair_batch<MODE, C, true><<<grid, W / 4 / C, smem, s>>>(p, st, sl, b, W, phase);
-    else k_swept_ks_pair_batch<MODE, C, false><<<grid, W / 4 / C, smem, s>>>(p, st, sl, b, W, phase);
+    if (p.ks_form == KS_POW2) return launch_dependent(k_swept_ks_pair_batch<MODE, C, true>, grid, W / 4 / C, smem, s, p, st, sl, b, W, phase);
+    return launch_dependent(k_swept_ks_pair_batch<MODE, C, false>, grid, W / 4 / C, smem, s, p, st, sl, b, W, phase);
 }
 template <int C>
 inline cudaError_t launch_ks_pair_batch(const Params<float> &p, int mode, int phase, float *st, float *sl,
                                         const BatchDev &b, int W, cudaStream_t s) {
     switch (mode) {
-    case MODE_UP: launch_ks_pair_batch_mode<MODE_UP, C>(p, st, sl, b, W, phase, s); break;
-    case MODE_DIAMOND: launch_ks_pair_batch_mode<MODE_DIAMOND, C>(p, st, sl, b, W, phase, s); break;
-    default: launch_ks_pair_batch_mode<MODE_DOWN, C>(p, st, sl, b, W, phase, s); break;
+    case MODE_UP: return launch_ks_pair_batch_mode<MODE_UP, C>(p, st, sl, b, W, phase, s);
+    case MODE_DIAMOND: return launch_ks_pair_batch_mode<MODE_DIAMOND, C>(p, st, sl, b, W, phase, s);
+    default: return launch_ks_pair_batch_mode<MODE_DOWN, C>(p, st, sl, b, W, phase, s);
     }
-    return cudaGetLastError();
 }
 #endif  // SW_KS_DIVIDE_TU
 
