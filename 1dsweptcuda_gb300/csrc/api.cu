@@ -103,7 +103,7 @@ struct Segment {
 struct Plan {
     bool swept = false;
     std::vector<Segment> segs;
-    int64_t remainder = 0;  // SW_TIME_STEPS swept: classic steps after the last segment
+    int64_t remainder = 0;  // SW_TIME_STEPS swept: time steps after the last segment (Runner::tail)
     int down_phase = 0;     // swept, SW_TIME_STEPS: phase of the final down-triangle
     double t_final = 0;
     int64_t steps = 0;
@@ -286,6 +286,18 @@ struct Runner {
         return rc;
     }
 
+    // the steps after the last whole cycle: narrower cycles (tail_tile), then classic
+    int tail(int64_t rem) {
+        const int64_t nx = cfg.nx;
+        while (const int w = host_tile ? 0 : tail_tile(*ops, (cfg.flags & SW_FLAG_KS_DIVIDE) != 0, W, nx, rem)) {
+            SW_CUDA(ctx, ops->swept(&p, MODE_UP, 0, cur, ctx->d_slots, nx, w, 0, s));
+            SW_CUDA(ctx, ops->swept(&p, MODE_DOWN, 1, cur, ctx->d_slots, nx, w, 0, s));
+            launches += 2;
+            rem -= w / (2 * ops->R * ops->S);
+        }
+        return classic_steps(rem);
+    }
+
     // cur back into the primary state buffer (Heat classic leaves it in alt after odd counts)
     int settle(void *primary) {
         if (cur != primary) {
@@ -392,7 +404,7 @@ int run_impl(sw_ctx *ctx, const sw_config &c, const void *ic_host, void *final_h
         }
     }
     if (pl.remainder) {
-        rc = r.classic_steps(pl.remainder);
+        rc = r.tail(pl.remainder);
         if (rc) return rc;
     }
     rc = r.settle(primary);
@@ -655,7 +667,14 @@ int sw_plan(const sw_config *cfg, sw_plan_info *out, double *snap_t, int64_t *sn
             ++k;
         }
     }
-    launches += pl.remainder * ops->S;
+    int64_t rem = pl.remainder;
+    while (const int w = (cfg->flags & SW_FLAG_HOST_TILE)
+                             ? 0
+                             : tail_tile(*ops, (cfg->flags & SW_FLAG_KS_DIVIDE) != 0, W, cfg->nx, rem)) {
+        launches += 2;
+        rem -= w / (2 * ops->R * ops->S);
+    }
+    launches += rem * ops->S;
     out->n_snapshots = k;
     out->launches = launches;
     return SW_OK;

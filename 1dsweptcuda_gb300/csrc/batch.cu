@@ -98,7 +98,7 @@ int ensure_tables(sw_ctx *ctx, int32_t n, const int64_t *nx, int W) {
         while (group > 1 && (nx[d] / W) % group != 0) group >>= 1;
     int32_t vec4 = 1;
     for (int32_t d = 0; d < n; ++d) vec4 = vec4 && nx[d] % 4 == 0;
-    bt.dev = BatchDev{d_dom, d_off, d_tile0, d_blk, tiles, cells, n, W ? group : 1, vec4};
+    bt.dev = BatchDev{d_dom, d_off, d_tile0, d_blk, tiles, cells, n, W ? group : 1, vec4, 1};
     bt.nx.assign(nx, nx + n);
     bt.W = W;
     if (ctx->graph.exec) {  // the tables moved: a cached graph may point at the old ones
@@ -130,7 +130,8 @@ int enqueue(sw_ctx *ctx, const Ops *ops, const Params<T> &p, const sw_config &c,
         return SW_OK;
     }
     const int64_t q = W / (2 * ops->R * ops->S);
-    const int64_t full = n / q, rem = n - full * q;
+    const int64_t full = n / q;
+    int64_t rem = n - full * q;
     if (full >= 1) {
         if (c.alg == SW_ALG_VARIANT) {
             SW_CUDA(ctx, ops->batch_persistent(&p, state, ctx->d_slots, b, ctx->d_flags, ctx->d_status, W, threads,
@@ -143,6 +144,16 @@ int enqueue(sw_ctx *ctx, const Ops *ops, const Params<T> &p, const sw_config &c,
             SW_CUDA(ctx, ops->batch_swept(&p, MODE_DOWN, (int)(full & 1), state, ctx->d_slots, b, W, threads, s));
             *launches += full + 1;
         }
+    }
+    // narrower cycles for the steps left over (tail_tile), on the tables of width W
+    while (const int w = tail_tile(*ops, (c.flags & SW_FLAG_KS_DIVIDE) != 0, W, b->n_cells, rem)) {
+        BatchDev nb = *b;
+        nb.split = W / w;
+        nb.n_tiles *= nb.split;
+        SW_CUDA(ctx, ops->batch_swept(&p, MODE_UP, 0, state, ctx->d_slots, &nb, w, 0, s));
+        SW_CUDA(ctx, ops->batch_swept(&p, MODE_DOWN, 1, state, ctx->d_slots, &nb, w, 0, s));
+        *launches += 2;
+        rem -= w / (2 * ops->R * ops->S);
     }
     void *cur = state, *alt = ctx->d_work;
     for (int64_t i = 0; i < rem; ++i) {

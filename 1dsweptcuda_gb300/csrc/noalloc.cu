@@ -84,12 +84,18 @@ int run(const sw_config &c, void *state, cudaStream_t s) {
     sw_constants_of(&c, &k);
     const Params<T> p = make_params<T>(c, k);
     const int64_t q = W / (2 * ops->R * ops->S);
-    const int64_t full = c.n_steps / q, rem = c.n_steps - full * q;
+    const int64_t full = c.n_steps / q;
+    int64_t rem = c.n_steps - full * q;
     if (full >= 1) {
         if (ops->swept(&p, MODE_UP, 0, state, slots, nx, W, c.threads, s) != cudaSuccess) return SW_ERR_CUDA;
         for (int64_t d = 1; d < full; ++d)
             if (ops->swept(&p, MODE_DIAMOND, (int)(d & 1), state, slots, nx, W, c.threads, s) != cudaSuccess) return SW_ERR_CUDA;
         if (ops->swept(&p, MODE_DOWN, (int)(full & 1), state, slots, nx, W, c.threads, s) != cudaSuccess) return SW_ERR_CUDA;
+    }
+    while (const int w = tail_tile(*ops, (c.flags & SW_FLAG_KS_DIVIDE) != 0, W, nx, rem)) {
+        if (ops->swept(&p, MODE_UP, 0, state, slots, nx, w, 0, s) != cudaSuccess) return SW_ERR_CUDA;
+        if (ops->swept(&p, MODE_DOWN, 1, state, slots, nx, w, 0, s) != cudaSuccess) return SW_ERR_CUDA;
+        rem -= w / (2 * ops->R * ops->S);
     }
     void *cur = state, *alt = work;
     for (int64_t i = 0; i < rem; ++i) {

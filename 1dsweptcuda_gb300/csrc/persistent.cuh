@@ -304,12 +304,12 @@ __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PA
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     const int64_t g = blockIdx.x;
-    const int d = b.tile_dom[g];
+    const int d = b.tile_dom[g / b.split];
     const int64_t off = b.off[d];
     Params<T> q = p;
     q.nx = b.off[d + 1] - off;
     swept_tile<P, T, MODE, PATH>(q, state + off, slots + 2 * off, reinterpret_cast<T *>(sw_smem), W, phase,
-                           g - b.tile0[d]);
+                           g - b.tile0[d] * b.split);
 }
 
 // G consecutive tiles of one domain per block (one cell per thread), as
@@ -322,12 +322,12 @@ __global__ void __launch_bounds__(1024, 2)
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     const int64_t g0 = G * (int64_t)blockIdx.x;
-    const int d = b.tile_dom[g0];
+    const int d = b.tile_dom[g0 / b.split];
     const int64_t off = b.off[d];
     Params<T> q = p;
     q.nx = b.off[d + 1] - off;
     swept_tile_group<P, T, MODE, G, PATH>(q, state + off, slots + 2 * off, reinterpret_cast<T *>(sw_smem), W, phase,
-                                          g0 - b.tile0[d]);
+                                          g0 - b.tile0[d] * b.split);
 }
 
 // Classic step of an ensemble, one cell per thread, kClassicBlock threads per

@@ -44,6 +44,7 @@ struct BatchDev {
     int32_t n_dom;
     int32_t group;  // the largest of 1, 2, 4 that divides every domain's tile count
     int32_t vec4;   // every domain length is a multiple of 4
+    int32_t split;  // the launch's tiles are 1/split of the tables' (tail_tile)
 };
 constexpr int kClassicBlock = 256;  // threads (= cells) per block of the ensemble classic kernel
 
@@ -84,6 +85,26 @@ struct Ops {
     cudaError_t (*batch_persistent)(const void *params, void *state, void *slots, const void *batch, unsigned *flags,
                                     int *status, int W, int threads, int64_t n_diamonds, cudaStream_t s);
 };
+
+// The tile width of one more swept cycle (an up- and a down-triangle, two
+// launches) that takes up to `rem` time steps left over after a run's whole
+// cycles of width W, or 0: classic steps, S launches each, for the rest.  A width
+// that divides W divides every domain of the run, and every (cell, sub-step)
+// value is the same whatever tile it is computed in.
+// A narrow cycle beats its classic steps where those are bound by launches and
+// memory: us per step at 2^20 and 2^22 cells, cycle against classic: Heat FP32 128
+// cells 1.5 and 4.8 against 1.8 and 5.0, 512 cells 0.9 and 3.1; KS FP32 128 cells
+// 3.0 and 9.3 against 4.1 and 10.9, 512 cells 1.9 and 6.1; Heat FP64 128 cells 6.3
+// and 24 against 7.3 and 25.  64 cells lose there (Heat FP32 2.8 and 10), but not
+// on small domains (4096 cells: 0.8 against 1.7).  FP64 KS and Euler are bound by
+// arithmetic, which classic wastes none of (KS FP64 128 cells 52 against 49).
+inline int tail_tile(const Ops &ops, bool divide, int W, int64_t cells, int64_t rem) {
+    if (divide || ops.problem == SW_EULER || (ops.problem == SW_KS && ops.prec == 8)) return 0;
+    const int least = cells <= ((int64_t)1 << 18) ? 64 : 128;
+    for (int k = 2; W / k >= least; ++k)
+        if (W % (32 * k) == 0 && W / k / (2 * ops.R * ops.S) <= rem) return W / k;
+    return 0;
+}
 
 // The hybrid variant's host tile (host_tile.cu): the wrapping phase-1 tile of
 // a domain computed on the CPU from its two slots (sl: the last half-tile's,

@@ -210,9 +210,9 @@ __global__ void __launch_bounds__(256 / C, (C == 2 ? 8 : 5))
     wait_for_previous_launch();
     const int64_t g0 = 2 * (int64_t)blockIdx.x, g1 = g0 + 1 < b.n_tiles ? g0 + 1 : g0;
     auto tile = [&](int64_t g) {
-        const int d = b.tile_dom[g];
+        const int d = b.tile_dom[g / b.split];
         const int64_t off = b.off[d];
-        return pair_tile(state + off, slots + 2 * off, W, phase, g - b.tile0[d], b.off[d + 1] - off);
+        return pair_tile(state + off, slots + 2 * off, W, phase, g - b.tile0[d] * b.split, b.off[d + 1] - off);
     };
     ks_pair_block<MODE, C, POW2>(p, tile(g0), tile(g1), reinterpret_cast<float2 *>(sw_smem), W);
 }

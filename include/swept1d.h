@@ -69,7 +69,8 @@ enum sw_bc {
 
 enum sw_time_mode {
     SW_TIME_REFERENCE = 0, /* the reference wrappers' t_eq bookkeeping from dt, tf, freq */
-    SW_TIME_STEPS = 1      /* exactly n_steps time steps (swept finishes the remainder classically) */
+    SW_TIME_STEPS = 1      /* exactly n_steps time steps (swept takes the steps after its last whole cycle in
+                              narrower cycles and classic steps) */
 };
 
 /* sw_config.flags */
