@@ -502,10 +502,11 @@ int sw_ctx_destroy(sw_ctx *c) {
     if (!c) return SW_ERR_ARG;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    void *bufs[] = {c->d_state, c->d_work, c->d_slots, c->d_io, c->d_flags, c->d_status, c->d_w2p, c->d_judge};
+    void *bufs[] = {c->d_state, c->d_work, c->d_slots, c->d_io, c->d_flags, c->d_status, c->d_fwd, c->d_judge};
     for (void *b : bufs)
         if (b) cudaFree(b);
     if (c->h_pin) cudaFreeHost(c->h_pin);
+    if (c->h_fwd_status) cudaFreeHost(c->h_fwd_status);
     if (c->h_tile) cudaFreeHost(c->h_tile);
     if (c->tile_ready) cudaEventDestroy(c->tile_ready);
     if (c->batch.d_tables) cudaFree(c->batch.d_tables);

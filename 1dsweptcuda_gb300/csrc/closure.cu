@@ -2,11 +2,15 @@
 // kernel 5, GELU, circular padding per domain) that corrects a coarse KS step.
 // Parameters are FP32 masters rounded to BF16 for the forward pass.  The
 // 32 -> 32 layer -- 94 % of the work -- runs on the tensor cores
-// (mma.sync.m16n8k16, BF16 operands, FP32 accumulation) forward and backward;
+// (tcgen05.mma in the forward pass, mma.sync.m16n8k16 in the backward pass; BF16
+// operands, FP32 accumulation);
 // the 1 -> 32 and 32 -> 1 layers run in FP32 on the CUDA cores with the
 // BF16-rounded weights.  oracle/closure.py restates the same arithmetic.
 //
-// Tiles: a block produces TOUT = 128 consecutive outputs of one domain.  In
+// The forward pass alone (inference, the coarse step) is closure_fwd.cuh; this
+// file has the backward pass, training and the certified adaptive run.
+//
+// Tiles of the backward pass: a block takes TOUT = 128 consecutive outputs of one domain.  In
 // tile coordinates (x0 = first output):
 //   us[j] = u[x0 - 6 + j],        j < 152
 //   a1[r] : position x0 - 4 + r,  r < 148  (z1 = w1 * us[r .. r+4] + b1)
@@ -60,27 +64,26 @@ __device__ __forceinline__ float tanh_sfu(float x) {
     asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-__device__ __forceinline__ float gelu(float x) {  // x/2 + (x/2) t, the operations of gelu2 below
+__device__ __forceinline__ float gelu(float x) {  // x/2 + (x/2) t
     const float t = tanh_sfu((kGeluC * x) * fmaf(kGeluA, x * x, 1.0f));
     const float hx = 0.5f * x;
     return fmaf(hx, t, hx);
 }
-// Two GELUs with paired FP32 instructions (one f32x2 instruction does the
-// arithmetic of two lanes' worth: the forward step is bound by instruction
-// issue).  Each component is gelu of that component, operation for operation.
 __device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 gelu2(float2 x) {
-    const float2 inner = __ffma2_rn(f2(kGeluA), __fmul2_rn(x, x), f2(1.0f));
-    const float2 arg = __fmul2_rn(__fmul2_rn(f2(kGeluC), x), inner);
-    const float2 hx = __fmul2_rn(f2(0.5f), x);
-    return __ffma2_rn(hx, make_float2(tanh_sfu(arg.x), tanh_sfu(arg.y)), hx);
-}
 __device__ __forceinline__ float gelu_grad(float x) {
     const float x2 = x * x;
     const float t = tanh_sfu(kGeluC * x * fmaf(kGeluA, x2, 1.0f));
     return fmaf(0.5f * x * (1.0f - t * t), kGeluC * fmaf(3.0f * kGeluA, x2, 1.0f), 0.5f * (1.0f + t));
 }
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
+}  // namespace cl
+}  // namespace sw
+
+#include "closure_fwd.cuh"
+
+namespace sw {
+namespace cl {
+
 __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
@@ -96,43 +99,26 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// Shared memory of a tile.  The forward kernels allocate only the part up to
-// z2 (smem_fwd_bytes); the backward kernel also keeps the pre-activations.
+// Shared memory of a tile.
 struct Smem {
     float us[NU];
     float w1[CH * KW], b1[CH], b2[CH], w3[CH * KW], b3, scale;
     __nv_bfloat16 a1[NA1 * LDB];                   // layer-1 activations, BF16 (the MMA A operand)
     alignas(16) __nv_bfloat16 w2[KW * CH * LDB];   // w2[t][o][i], i contiguous (the MMA B operand)
-    float pred[TOUT + 4];                          // k_step: the KS predictor on x0-2 .. x0+TOUT+1
-    float p3[KW * NA2];                            // forward: p3[t][r] = sum_i w3[i][t] a2[r][i]
-    float a2[NA2 * LDF];                           // layer-2 activations gelu(z2) (backward only)
-    float z2[NA2 * LDF];                           // layer-2 pre-activations (backward only)
-    float z1[NA1 * LDF];                           // layer-1 pre-activations (backward only)
+    float a2[NA2 * LDF];                           // layer-2 activations gelu(z2)
+    float z2[NA2 * LDF];                           // layer-2 pre-activations
+    float z1[NA1 * LDF];                           // layer-1 pre-activations
 };
-constexpr int W2P_WORDS = KW * CH * LDB * 2 / 16;  // the staged w2 in 16-byte words
 
-// theta's w2 (flat [o][i][t], FP32) -> BF16 in the shared-memory layout [t][o][i]
-// (row stride LDB; the padding columns are zero), once per call of the
-// forward kernels instead of once per block.
-__global__ void k_pack_w2(const float *__restrict__ theta, __nv_bfloat16 *__restrict__ w2p) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= KW * CH * LDB) return;
-    const int t = k / (CH * LDB), o = (k / LDB) % CH, i = k % LDB;
-    w2p[k] = __float2bfloat16_rn(i < CH ? theta[OW2 + (o * CH + i) * KW + t] : 0.0f);
-}
-
-// Load the tile's inputs (periodic within the domain) and, unless `weights`
-// is false, the weights; w2 from the staged copy w2p (16-byte words) when
-// given, else from theta.
+// Load the tile's inputs (periodic within the domain) and the weights.
 __device__ void load_tile(Smem &s, const float *__restrict__ theta, const float *__restrict__ u, int64_t n,
-                          int64_t x0, const uint4 *__restrict__ w2p = nullptr, bool weights = true) {
+                          int64_t x0) {
     for (int j = threadIdx.x; j < NU; j += blockDim.x) {
         int64_t q = x0 - 6 + j;
         q %= n;
         if (q < 0) q += n;
         s.us[j] = u[q];
     }
-    if (!weights) return;
     for (int i = threadIdx.x; i < CH * KW; i += blockDim.x) {
         s.w1[i] = bf16r(theta[OW1 + i]);
         s.w3[i] = bf16r(theta[OW3 + i]);
@@ -145,11 +131,6 @@ __device__ void load_tile(Smem &s, const float *__restrict__ theta, const float 
         s.b3 = theta[OB3];
         s.scale = theta[OSCALE];
     }
-    if (w2p) {
-        uint4 *dst = reinterpret_cast<uint4 *>(s.w2);
-        for (int k = threadIdx.x; k < W2P_WORDS; k += blockDim.x) dst[k] = w2p[k];
-        return;
-    }
     // w2 flat is [o][i][t]; smem is [t][o][i]
     for (int k = threadIdx.x; k < CH * CH * KW; k += blockDim.x) {
         const int o = k / (CH * KW), i = (k / KW) % CH, t = k % KW;
@@ -157,14 +138,8 @@ __device__ void load_tile(Smem &s, const float *__restrict__ theta, const float 
     }
 }
 
-// Layers 1 and 2 of the forward pass.  TRAIN: a1 (BF16), a2 = gelu(z2) (FP32)
-// and the pre-activations z1, z2 for the backward pass.  Otherwise layer 3's
-// per-row tap sums p3[t][r] = sum_i w3[i][t] gelu(z2[r][i]) are formed in the
-// MMA epilogue, so a2 is never stored: each lane holds 8 channels of rows r
-// and r + 8, dots them with w3 for the five taps, and the four lanes of a row
-// add their sums by shuffles (output q is then b3 + sum_t p3[t][q + t]).
-// Requires load_tile and a barrier first.
-template <bool TRAIN>
+// Layers 1 and 2 of the forward pass: a1 (BF16), a2 = gelu(z2) (FP32) and the
+// pre-activations z1, z2 for the backward pass.  Requires load_tile and a barrier first.
 __device__ void forward_12(Smem &s) {
     {
         // lane = output channel o; each warp a contiguous run of rows, with o's
@@ -178,26 +153,6 @@ __device__ void forward_12(Smem &s) {
         for (int t = 0; t < KW; ++t) w[t] = s.w1[o * KW + t];
         const float b = s.b1[o];
         int r = r0;
-        if constexpr (!TRAIN) {
-            // two rows per iteration as f32x2 pairs: window v[0..5] = inputs r .. r+5
-            float v[KW + 1];
-            if (r0 < r1) {
-#pragma unroll
-                for (int t = 0; t < KW - 1; ++t) v[t + 2] = s.us[r0 + t];
-            }
-            for (; r + 1 < r1; r += 2) {
-#pragma unroll
-                for (int t = 0; t < KW - 1; ++t) v[t] = v[t + 2];
-                v[KW - 1] = s.us[r + KW - 1];
-                v[KW] = s.us[r + KW];
-                float2 z = f2(b);
-#pragma unroll
-                for (int t = 0; t < KW; ++t) z = __ffma2_rn(f2(w[t]), make_float2(v[t], v[t + 1]), z);
-                const float2 g = gelu2(z);
-                s.a1[r * LDB + o] = __float2bfloat16_rn(g.x);
-                s.a1[(r + 1) * LDB + o] = __float2bfloat16_rn(g.y);
-            }
-        }
         if (r < r1) {
 #pragma unroll
             for (int t = 0; t < KW - 1; ++t) u[t + 1] = s.us[r + t];
@@ -209,7 +164,7 @@ __device__ void forward_12(Smem &s) {
             float z = b;
 #pragma unroll
             for (int t = 0; t < KW; ++t) z = fmaf(w[t], u[t], z);
-            if (TRAIN) s.z1[r * LDF + o] = z;
+            s.z1[r * LDF + o] = z;
             s.a1[r * LDB + o] = __float2bfloat16_rn(gelu(z));
         }
     }
@@ -236,7 +191,7 @@ __device__ void forward_12(Smem &s) {
             }
         }
         const int r0 = p0 + g, r1 = p0 + g + 8;
-        if constexpr (TRAIN) {
+        {
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
                 const int o = nt * 8 + 2 * q;
@@ -255,52 +210,12 @@ __device__ void forward_12(Smem &s) {
                     s.a2[r1 * LDF + o + 1] = gelu(z3);
                 }
             }
-        } else {
-            // GELU on channel pairs (o, o+1) of a row, the tap sums on row pairs (r0, r1)
-            float2 pr[KW];
-#pragma unroll
-            for (int t = 0; t < KW; ++t) pr[t] = f2(0.0f);
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int o = nt * 8 + 2 * q;
-                const float2 bias = make_float2(s.b2[o], s.b2[o + 1]);
-                const float2 g0 = gelu2(__fadd2_rn(make_float2(acc[nt][0], acc[nt][1]), bias));  // row r0
-                const float2 g1 = gelu2(__fadd2_rn(make_float2(acc[nt][2], acc[nt][3]), bias));  // row r1
-                const float2 c0 = make_float2(g0.x, g1.x), c1 = make_float2(g0.y, g1.y);         // channel o, o+1
-#pragma unroll
-                for (int t = 0; t < KW; ++t) {
-                    pr[t] = __ffma2_rn(f2(s.w3[o * KW + t]), c0, pr[t]);
-                    pr[t] = __ffma2_rn(f2(s.w3[(o + 1) * KW + t]), c1, pr[t]);
-                }
-            }
-#pragma unroll
-            for (int t = 0; t < KW; ++t) {
-                pr[t].x += __shfl_xor_sync(0xffffffffu, pr[t].x, 1);
-                pr[t].y += __shfl_xor_sync(0xffffffffu, pr[t].y, 1);
-                pr[t].x += __shfl_xor_sync(0xffffffffu, pr[t].x, 2);
-                pr[t].y += __shfl_xor_sync(0xffffffffu, pr[t].y, 2);
-            }
-            if (q == 0) {
-#pragma unroll
-                for (int t = 0; t < KW; ++t) {
-                    if (r0 < NA2) s.p3[t * NA2 + r0] = pr[t].x;
-                    if (r1 < NA2) s.p3[t * NA2 + r1] = pr[t].y;
-                }
-            }
         }
     }
     __syncthreads();
 }
 
-// Layer 3 for output q from the epilogue's tap sums: b3 + sum_t p3[t][q + t].
-__device__ __forceinline__ float layer3_sums(const Smem &s, int q) {
-    float d = 0.0f;
-#pragma unroll
-    for (int t = 0; t < KW; ++t) d += s.p3[t * NA2 + q + t];
-    return d + s.b3;
-}
-
-// Layer 3 for output q (backward pass, from the stored a2): b3 + sum_{t,i} w3[i][t] * a2[q + t][i].
+// Layer 3 for output q: b3 + sum_{t,i} w3[i][t] * a2[q + t][i].
 __device__ __forceinline__ float layer3(const Smem &s, int q) {
     float d = 0.0f;
 #pragma unroll
@@ -311,47 +226,6 @@ __device__ __forceinline__ float layer3(const Smem &s, int q) {
 }
 
 // ---------------------------------------------------------------- kernels
-// delta = f(u) for every cell of n_dom domains of n cells (n a multiple of TOUT).
-__global__ void __launch_bounds__(THREADS) k_infer(const float *__restrict__ theta, const uint4 *__restrict__ w2p,
-                                                   const float *__restrict__ u, float *__restrict__ delta, int64_t n,
-                                                   int64_t tiles_per_dom) {
-    extern __shared__ __align__(16) unsigned char raw[];
-    Smem &s = *reinterpret_cast<Smem *>(raw);
-    const int64_t dom = blockIdx.x / tiles_per_dom, x0 = (blockIdx.x % tiles_per_dom) * TOUT;
-    const float *ud = u + dom * n;
-    load_tile(s, theta, ud, n, x0, w2p);
-    __syncthreads();
-    forward_12<false>(s);
-    for (int q = threadIdx.x; q < TOUT; q += blockDim.x) delta[dom * n + x0 + q] = s.scale * layer3_sums(s, q);
-}
-
-// One coarse KS step fused with the closure: u_out = classic KS step(u_in) + f(u_in).
-// The KS predictor/corrector reads u_in on [x0-4, x0+TOUT+4) from the same tile.
-__global__ void __launch_bounds__(THREADS) k_step(const float *__restrict__ theta, const uint4 *__restrict__ w2p,
-                                                  const Params<float> pk, const float *__restrict__ u,
-                                                  float *__restrict__ out, int64_t n, int64_t tiles_per_dom,
-                                                  int use_closure) {
-    extern __shared__ __align__(16) unsigned char raw[];
-    Smem &s = *reinterpret_cast<Smem *>(raw);
-    const int64_t dom = blockIdx.x / tiles_per_dom, x0 = (blockIdx.x % tiles_per_dom) * TOUT;
-    wait_for_previous_launch();
-    load_tile(s, theta, u + dom * n, n, x0, w2p, use_closure != 0);  // theta may be null without the closure
-    __syncthreads();
-    if (use_closure) forward_12<false>(s);
-    // predictor on positions x0-2 .. x0+TOUT+1 (us index 4 .. TOUT+7)
-    for (int j = threadIdx.x; j < TOUT + 4; j += blockDim.x) {
-        const int c = j + 4;
-        s.pred[j] = ks_predict(pk, s.us[c - 2], s.us[c - 1], s.us[c], s.us[c + 1], s.us[c + 2]);
-    }
-    __syncthreads();
-    for (int q = threadIdx.x; q < TOUT; q += blockDim.x) {
-        const int c = q + 6, j = q + 2;  // us index of x0+q; predictor index of x0+q
-        float v = ks_correct(pk, s.us[c], s.pred[j - 2], s.pred[j - 1], s.pred[j], s.pred[j + 1], s.pred[j + 2]);
-        if (use_closure) v += s.scale * layer3_sums(s, q);
-        out[dom * n + x0 + q] = v;
-    }
-}
-
 // Loss and parameter gradients (forward + backward), summed over the tiles a
 // block visits into its row of `partial` ([gridDim.x][NPARAM + 1], last = loss).
 // The loss is on the scaled defect: L = wpt * sum (net(u) - target / s)^2,
@@ -378,7 +252,7 @@ __global__ void __launch_bounds__(THREADS) k_grad(const float *__restrict__ thet
         const int64_t dom = rows ? rows[b] : b;  // minibatch row -> sample
         load_tile(s, theta, u + dom * n, n, x0);
         __syncthreads();
-        forward_12<true>(s);
+        forward_12(s);
         // delta, dL/ddelta, loss, dW3, db3
         for (int q = threadIdx.x; q < TOUT; q += blockDim.x) {
             const float d = layer3(s, q);
@@ -580,7 +454,6 @@ __global__ void __launch_bounds__(256) k_rel_l2(const float *__restrict__ a, con
 }
 
 constexpr size_t smem_bytes() { return sizeof(Smem); }
-constexpr size_t smem_fwd_bytes() { return offsetof(Smem, a2); }
 
 }  // namespace cl
 }  // namespace sw
@@ -603,11 +476,7 @@ cudaError_t allow_smem() {
     if (e != cudaSuccess) return e;
     const uint64_t bit = (dev >= 0 && dev < 64) ? (uint64_t(1) << dev) : 0;
     if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
-    e = cudaFuncSetAttribute(cl::k_infer, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::smem_fwd_bytes());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cl::k_step, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::smem_fwd_bytes());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cl::k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::smem_bytes());
+    e = cudaFuncSetAttribute(cl::k_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl::smem_bytes());
     if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
     return e;
 }
@@ -621,14 +490,44 @@ int after_legacy(sw_ctx *ctx) {
     return SW_OK;
 }
 
-// Stage theta's layer-2 weights for the forward kernels (stream-ordered before them).
-int stage_w2(sw_ctx *ctx, const float *theta, const uint4 **w2p) {
-    if (!ctx->d_w2p) SW_CUDA(ctx, cudaMalloc(&ctx->d_w2p, (size_t)cl::W2P_WORDS * 16));
-    const int total = cl::KW * cl::CH * cl::LDB;
-    cl::k_pack_w2<<<(total + 255) / 256, 256, 0, ctx->stream>>>(theta, static_cast<__nv_bfloat16 *>(ctx->d_w2p));
+// Stage theta for the forward kernels (stream-ordered before them).
+int stage_weights(sw_ctx *ctx, const float *theta) {
+    if (!ctx->d_fwd) SW_CUDA(ctx, cudaMalloc(&ctx->d_fwd, sizeof(cl::FwdWeights)));
+    if (!ctx->h_fwd_status) {
+        SW_CUDA(ctx, cudaMallocHost(&ctx->h_fwd_status, sizeof(int)));
+        *ctx->h_fwd_status = 0;
+    }
+    cl::k_pack_weights<<<(cl::CH * cl::CH * cl::KW + 255) / 256, 256, 0, ctx->stream>>>(
+        theta, static_cast<cl::FwdWeights *>(ctx->d_fwd));
     SW_CUDA(ctx, cudaGetLastError());
-    *w2p = static_cast<const uint4 *>(ctx->d_w2p);
     return SW_OK;
+}
+
+// One forward launch over n_dom domains of n cells.  Dependent launches read the staged weights before they wait for
+// the launch before them, so the first launch after stage_weights is an ordinary one.
+template <bool STEP>
+cudaError_t launch_forward(sw_ctx *ctx, bool dependent, const Params<float> &p, const float *u, float *out, int32_t n_dom,
+                           int64_t n) {
+    const int n_out = n == 128 ? 128 : cl::FWD_OUT;
+    const uint32_t per_dom = (uint32_t)((n + n_out - 1) / n_out), tiles = per_dom * (uint32_t)n_dom;
+    int sms = 0;
+    cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    if (e != cudaSuccess) return e;
+    const unsigned grid = std::min<unsigned>(tiles, (unsigned)(sms * cl::FWD_BLOCKS));
+    const cl::FwdWeights *w = static_cast<const cl::FwdWeights *>(ctx->d_fwd);
+    if (dependent)
+        return launch_dependent(cl::k_forward<STEP>, grid, cl::FWD_THREADS, 0, ctx->stream, w, p, u, out, n, per_dom, tiles,
+                                n_out, ctx->h_fwd_status);
+    cl::k_forward<STEP><<<grid, cl::FWD_THREADS, 0, ctx->stream>>>(w, p, u, out, n, per_dom, tiles, n_out,
+                                                                    ctx->h_fwd_status);
+    return cudaGetLastError();
+}
+
+// After the forward launches have completed.
+int forward_status(sw_ctx *ctx) {
+    if (!ctx->h_fwd_status || !*(volatile int *)ctx->h_fwd_status) return SW_OK;
+    *ctx->h_fwd_status = 0;
+    return fail(ctx, SW_ERR_TIMEOUT, "closure kernel: a tensor-core wait ran out");
 }
 
 }  // namespace
@@ -641,16 +540,10 @@ int sw_closure_infer(sw_ctx *ctx, const float *theta, const float *u, float *del
     if (!theta || !u || !delta) return SW_ERR_ARG;
     SW_CUDA(ctx, cudaSetDevice(ctx->device));
     if ((rc = after_legacy(ctx)) != SW_OK) return rc;
-    SW_CUDA(ctx, allow_smem());
-    const int64_t tiles = n / cl::TOUT;
-    const uint4 *w2p = nullptr;
-    rc = stage_w2(ctx, theta, &w2p);
-    if (rc) return rc;
-    cl::k_infer<<<(unsigned)(tiles * n_dom), cl::THREADS, cl::smem_fwd_bytes(), ctx->stream>>>(theta, w2p, u, delta, n,
-                                                                                                tiles);
-    SW_CUDA(ctx, cudaGetLastError());
+    if ((rc = stage_weights(ctx, theta))) return rc;
+    SW_CUDA(ctx, launch_forward<false>(ctx, false, Params<float>{}, u, delta, n_dom, n));
     SW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return SW_OK;
+    return forward_status(ctx);
 }
 
 }  // extern "C"
@@ -672,18 +565,17 @@ int closure_enqueue(sw_ctx *ctx, const sw_config *coarse, const float *theta, fl
     const Params<float> p = make_params<float>(c, k);
     SW_CUDA(ctx, cudaSetDevice(ctx->device));
     if ((rc = after_legacy(ctx)) != SW_OK) return rc;
-    SW_CUDA(ctx, allow_smem());
     SW_CUDA(ctx, grow_dev(&ctx->d_work, &ctx->n_work, sizeof(float) * (size_t)n * n_dom));
     float *alt = static_cast<float *>(ctx->d_work), *cur = u;
-    const int64_t tiles = n / cl::TOUT;
-    const uint4 *w2p = nullptr;
-    if (use_closure) {
-        rc = stage_w2(ctx, theta, &w2p);
-        if (rc) return rc;
-    }
+    if (use_closure && (rc = stage_weights(ctx, theta))) return rc;
+    const uint32_t warps_per_dom = (uint32_t)(n / 128), warps = warps_per_dom * (uint32_t)n_dom;
+    constexpr uint32_t per_block = cl::PLAIN_THREADS / 32;
     for (int64_t i = 0; i < n_steps; ++i) {
-        SW_CUDA(ctx, launch_dependent(cl::k_step, (unsigned)(tiles * n_dom), cl::THREADS, cl::smem_fwd_bytes(), ctx->stream,
-                                      theta, w2p, p, cur, alt, n, tiles, use_closure));
+        if (use_closure)
+            SW_CUDA(ctx, launch_forward<true>(ctx, i > 0, p, cur, alt, n_dom, n));
+        else
+            SW_CUDA(ctx, launch_dependent(cl::k_plain_step, (warps + per_block - 1) / per_block, cl::PLAIN_THREADS, 0,
+                                          ctx->stream, p, cur, alt, n, warps_per_dom, warps));
         std::swap(cur, alt);
     }
     SW_CUDA(ctx, cudaGetLastError());
@@ -704,6 +596,7 @@ int sw_closure_step(sw_ctx *ctx, const sw_config *coarse, const float *theta, fl
     if (rc) return rc;
     SW_CUDA(ctx, cudaEventRecord(ctx->k1, ctx->stream));
     SW_CUDA(ctx, cudaEventSynchronize(ctx->k1));
+    if (const int st = forward_status(ctx)) return st;
     if (out) {
         float ms = 0;
         cudaEventElapsedTime(&ms, ctx->k0, ctx->k1);
@@ -899,6 +792,7 @@ int sw_closure_adaptive(sw_ctx *ctx, sw_ctx *judge, const sw_config *coarse, con
             if ((rc = rel(samp2, nullptr, 1))) return rc;
             SW_CUDA(ctx, cudaMemcpyAsync(h_err.data(), err, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, s));
             SW_CUDA(ctx, cudaStreamSynchronize(s));
+            if ((rc = forward_status(ctx))) return rc;
             double m0, m1, x0, x1;
             stats(0, &m0, &x0);
             stats(1, &m1, &x1);
@@ -916,6 +810,7 @@ int sw_closure_adaptive(sw_ctx *ctx, sw_ctx *judge, const sw_config *coarse, con
             if ((rc = rel(samp, nullptr, 1))) return rc;
             SW_CUDA(ctx, cudaMemcpyAsync(h_err.data(), err, sizeof(double) * 2 * m, cudaMemcpyDeviceToHost, s));
             SW_CUDA(ctx, cudaStreamSynchronize(s));
+            if ((rc = forward_status(ctx))) return rc;
             cur_slot = 0;
             alt_slot = 1;
         }

@@ -111,7 +111,8 @@ struct sw_ctx {
     unsigned *d_flags = nullptr;
     size_t n_flags = 0;
     int *d_status = nullptr;
-    void *d_w2p = nullptr;  // closure layer-2 weights, BF16, in the kernels' shared-memory layout
+    void *d_fwd = nullptr;        // closure weights in the forward kernels' layout
+    int *h_fwd_status = nullptr;  // pinned: a forward kernel's wait that ran out
     void *d_judge = nullptr;  // sw_closure_adaptive: the sample's rows, errors (run context) or fine shadow (judge)
     size_t n_judge = 0;
     void *h_pin = nullptr;
