@@ -14,14 +14,19 @@
 // rows shifted by a tap are the same planes 16 bytes on: the im2col is a start
 // address.  Layer 1 writes a plane per warp (consecutive lanes 16 bytes apart);
 // the epilogue reads a row of 32 sums per thread, so its tap sums need no
-// shuffles.  The arithmetic runs on channel pairs (f32x2); inputs are stored
-// twice, (u, u), the form those instructions read.
+// shuffles.  The arithmetic runs on channel pairs (f32x2).
 //
-// What bounds it: the FP32 and SFU pipes and instruction issue.  A cell takes 64
-// tanh, 16 per clock and SM.  Eight 128-thread blocks of 64 registers per SM
-// cover the MMA's latency and each other's barriers; each takes its tiles in a
-// stride of the grid, so weights and TMEM (32 columns) are set up once per block,
-// before the wait for the launch before it.
+// What bounds it: shared memory and latency.  A cell takes 64 tanh (16 per clock
+// and SM) and the MMAs read each row of a1 ten times, but with one tile at a time
+// most of shared memory's cycles went into the epilogue's weights, 32 lanes x 16
+// bytes a read although all lanes read the same.  So a block takes NT = 2 tiles
+// at a time where there are enough (the rule is at the launch), each weight read
+// serving both.  At 1024 domains of 1024 cells a step takes 102.5 us with
+// mma.sync, 54 us with one tile, 48.5 us with two (FP32 pipe 41 % busy, SFU 32 %,
+// tensor core 32 %, issue slots 49 %, shared memory 54 %); 4, 6 blocks per SM instead of 5:
+// 49.1, 49.9 us.  Blocks take their tiles in a stride of the grid, so weights and
+// TMEM are set up once per block, before the wait for the launch before it, and
+// the next tiles' inputs are fetched behind the work.
 //
 // The GELUs are kept doubled, 2 gelu(x) = x + x tanh(...), and the next layer's
 // weights halved: powers of two, exact in BF16 and FP32.
@@ -34,10 +39,9 @@
 namespace sw {
 namespace cl {
 
-constexpr int FWD_THREADS = 128, FWD_BLOCKS = 8;  // blocks per SM
+constexpr int FWD_THREADS = 128, FWD_BLOCKS = 5;  // blocks per SM
 constexpr int FWD_OUT = 124;                      // outputs per tile of a domain of more than 128 cells
 constexpr int FWD_PLANE = 136 * 16;               // bytes of one a1 plane (132 rows used)
-constexpr int FWD_TMEM = 32;                      // columns: 16 blocks of an SM fit its 512
 
 // The parameters in the layout of shared memory (k_pack_weights), halved as above.
 struct alignas(16) FwdWeights {
@@ -48,12 +52,13 @@ struct alignas(16) FwdWeights {
 };
 static_assert(sizeof(FwdWeights) % 16 == 0, "copied in 16-byte words");
 
+template <int NT>
 struct alignas(128) FwdSmem {
     FwdWeights w;
-    unsigned char a1[4 * FWD_PLANE];
-    float2 us[136];
-    float pred[128];    // KS predictor on x0-2 .. x0+125
-    float p3[KW][128];  // p3[t][r] = sum_i w3[i][t] gelu(z2[r][i])
+    unsigned char a1[NT][4 * FWD_PLANE];
+    float us[NT][136];
+    float pred[NT][128];    // KS predictor on x0-2 .. x0+125
+    float p3[NT][KW][128];  // p3[t][r] = sum_i w3[i][t] gelu(z2[r][i])
     uint64_t bar;
     uint32_t tmem;
 };
@@ -124,13 +129,15 @@ __device__ __forceinline__ bool umma_wait(uint64_t *bar, unsigned parity) {
 }
 
 // STEP: out = classic KS step(u) + scale net(u); else out = scale net(u).  Domains of n cells, tiles_per_dom tiles
-// of n_out outputs each (the last of a domain fewer).  A wait that runs out sets *status (pinned host memory).
-template <bool STEP>
+// of n_out outputs each (the last of a domain fewer); a block takes NT tiles at a time.  A wait that runs out sets
+// *status (pinned host memory).
+template <bool STEP, int NT>
 __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
     k_forward(const FwdWeights *__restrict__ weights, const Params<float> pk, const float *__restrict__ u,
               float *__restrict__ out, const int64_t n, const uint32_t tiles_per_dom, const uint32_t n_tiles,
               const int n_out, int *status) {
-    __shared__ FwdSmem s;
+    __shared__ FwdSmem<NT> s;
+    constexpr uint32_t TMEM_COLS = 32 * NT;  // the blocks that fit an SM's shared memory use at most 384 of its 512
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     {
         const uint4 *src = reinterpret_cast<const uint4 *>(weights);
@@ -139,7 +146,7 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
     }
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s.tmem)),
-                     "r"(FWD_TMEM)
+                     "r"(TMEM_COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
@@ -148,30 +155,44 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
     __syncthreads();
     tcgen05_after_sync();
     const uint32_t tmem = s.tmem;
-    const uint64_t da = umma_desc(smem_addr(s.a1), FWD_PLANE), db = umma_desc(smem_addr(s.w.w2), CH * 16);
     wait_for_previous_launch();
 
-    auto input = [&](uint32_t tile, int j) -> float {  // u at position x0 - 6 + j of the tile's domain, n >= 128 > j - 6 - 4
-        const uint32_t dom = tile / tiles_per_dom;
-        int64_t x = (int64_t)(tile - dom * tiles_per_dom) * n_out - 6 + j;
-        x += x < 0 ? n : 0;
-        x -= x >= n ? n : 0;
-        return u[(int64_t)dom * n + x];
-    };
-    float next = 0.0f, next_hi = 0.0f;
-    if (blockIdx.x < n_tiles) {
-        next = input(blockIdx.x, tid);
-        if (tid < 8) next_hi = input(blockIdx.x, 128 + tid);
-    }
-    unsigned parity = 0;
-    for (uint32_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-        s.us[tid] = f2(next);
-        if (tid < 8) s.us[128 + tid] = f2(next_hi);
-        __syncthreads();
-        if (n_tiles - tile > gridDim.x) {  // the next tile's inputs arrive behind this tile's work
-            next = input(tile + gridDim.x, tid);
-            if (tid < 8) next_hi = input(tile + gridDim.x, 128 + tid);
+    // the next tiles' inputs (positions x0 - 6 + tid and, for 8 threads, x0 + 122 + tid; n >= 128), and their
+    // place: row[h] the domain's first cell, at[h] this thread's output in the domain
+    float next[NT], next_hi[NT];
+    int64_t row[NT], at[NT], next_row[NT], next_at[NT];
+    auto fetch = [&](uint32_t first) {
+#pragma unroll
+        for (int h = 0; h < NT; ++h) {
+            const uint32_t tile = min(first + h, n_tiles - 1);  // past the last: its inputs again, its outputs dropped
+            const uint32_t dom = tile / tiles_per_dom;
+            next_row[h] = (int64_t)dom * n;
+            next_at[h] = (int64_t)(tile - dom * tiles_per_dom) * n_out + tid;
+            int64_t x = next_at[h] - 6;
+            x += x < 0 ? n : 0;
+            x -= x >= n ? n : 0;
+            next[h] = u[next_row[h] + x];
+            if (tid < 8) {
+                x = next_at[h] + 122;
+                x -= x >= n ? n : 0;
+                next_hi[h] = u[next_row[h] + x];
+            }
+            if (first + h >= n_tiles) next_at[h] = n;
         }
+    };
+    const uint32_t stride = gridDim.x * NT;
+    if (blockIdx.x * NT < n_tiles) fetch(blockIdx.x * NT);
+    unsigned parity = 0;
+    for (uint32_t first = blockIdx.x * NT; first < n_tiles; first += stride) {
+#pragma unroll
+        for (int h = 0; h < NT; ++h) {
+            s.us[h][tid] = next[h];
+            if (tid < 8) s.us[h][128 + tid] = next_hi[h];
+            row[h] = next_row[h];
+            at[h] = next_at[h];
+        }
+        __syncthreads();
+        if (n_tiles - first > stride) fetch(first + stride);  // arrives behind this tile's work
         // layer 1: a warp takes 8 channels (one plane) of all rows
         {
             float2 w[4][KW + 1];
@@ -185,12 +206,12 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
                     w[c][2 * k + 1] = make_float2(v.z, v.w);
                 }
             }
-            unsigned char *plane = s.a1 + warp * FWD_PLANE;
 #pragma unroll 1
-            for (int r = lane; r < 128; r += 32) {
+            for (int k = 0; k < 4 * NT; ++k) {
+                const int h = k >> 2, r = (k & 3) * 32 + lane;
                 float2 x[KW];
 #pragma unroll
-                for (int t = 0; t < KW; ++t) x[t] = s.us[r + t];
+                for (int t = 0; t < KW; ++t) x[t] = f2(s.us[h][r + t]);
                 __nv_bfloat162 a[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -199,61 +220,86 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
                     for (int t = 0; t < KW; ++t) z = __ffma2_rn(w[c][t], x[t], z);
                     a[c] = __float22bfloat162_rn(gelu2_doubled(z));
                 }
-                *reinterpret_cast<uint4 *>(plane + r * 16) = *reinterpret_cast<const uint4 *>(a);
+                *reinterpret_cast<uint4 *>(s.a1[h] + warp * FWD_PLANE + r * 16) = *reinterpret_cast<const uint4 *>(a);
             }
-            if (lane < 16) {  // rows 128 .. 131, a channel pair per lane
-                const int r = 128 + (lane >> 2), c = lane & 3;
+            if (lane < 16 * NT) {  // rows 128 .. 131, a channel pair per lane
+                const int h = lane >> 4, r = 128 + ((lane >> 2) & 3), c = lane & 3;
                 const float2 *wc = s.w.w1[warp * 4 + c];
                 float2 z = wc[KW];
 #pragma unroll
-                for (int t = 0; t < KW; ++t) z = __ffma2_rn(wc[t], s.us[r + t], z);
-                *reinterpret_cast<__nv_bfloat162 *>(plane + r * 16 + c * 4) = __float22bfloat162_rn(gelu2_doubled(z));
+                for (int t = 0; t < KW; ++t) z = __ffma2_rn(wc[t], f2(s.us[h][r + t]), z);
+                *reinterpret_cast<__nv_bfloat162 *>(s.a1[h] + warp * FWD_PLANE + r * 16 + c * 4) =
+                    __float22bfloat162_rn(gelu2_doubled(z));
             }
         }
-        if constexpr (STEP)
-            s.pred[tid] = ks_predict(pk, s.us[tid + 2].x, s.us[tid + 3].x, s.us[tid + 4].x, s.us[tid + 5].x, s.us[tid + 6].x);
+        if constexpr (STEP) {
+#pragma unroll
+            for (int h = 0; h < NT; ++h) {
+                const float *c = &s.us[h][tid + 4];
+                s.pred[h][tid] = ks_predict(pk, c[-2], c[-1], c[0], c[1], c[2]);
+            }
+        }
         fence_smem_for_bulk();  // a1 and the weights are read by the tensor core's copy path
         tcgen05_before_sync();
         __syncthreads();
         if (tid == 0) {
             tcgen05_after_sync();
 #pragma unroll
-            for (int k = 0; k < 2 * KW; ++k) {  // tap k / 2, input channels 16 (k % 2) on: descriptor offsets in 16 bytes
-                const int t = k >> 1, h = k & 1;
-                umma(tmem, da + t + h * (2 * FWD_PLANE / 16), db + t * (4 * CH) + h * (2 * CH), k > 0);
+            for (int h = 0; h < NT; ++h) {
+                const uint64_t da = umma_desc(smem_addr(s.a1[h]), FWD_PLANE), db = umma_desc(smem_addr(s.w.w2), CH * 16);
+#pragma unroll
+                for (int k = 0; k < 2 * KW; ++k) {  // tap k / 2, input channels 16 (k % 2) on: offsets in 16 bytes
+                    const int t = k >> 1, c = k & 1;
+                    umma(tmem + 32 * h, da + t + c * (2 * FWD_PLANE / 16), db + t * (4 * CH) + c * (2 * CH), k > 0);
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(&s.bar))
                          : "memory");
         }
         __syncwarp();
-        float v = 0.0f;
-        if constexpr (STEP)  // a domain of 128 cells wraps onto its own predictors
-            v = ks_correct(pk, s.us[tid + 6].x, s.pred[tid], s.pred[(tid + 1) & 127], s.pred[(tid + 2) & 127],
-                           s.pred[(tid + 3) & 127], s.pred[(tid + 4) & 127]);
+        float v[NT];
+#pragma unroll
+        for (int h = 0; h < NT; ++h) {
+            v[h] = 0.0f;
+            if constexpr (STEP) {  // a domain of 128 cells wraps onto its own predictors
+                const float *p = s.pred[h];
+                v[h] = ks_correct(pk, s.us[h][tid + 6], p[tid], p[(tid + 1) & 127], p[(tid + 2) & 127], p[(tid + 3) & 127],
+                                  p[(tid + 4) & 127]);
+            }
+        }
         const bool done = __all_sync(0xffffffffu, umma_wait(&s.bar, parity));
         if (done) {
             tcgen05_after_sync();
-            float2 sum[KW];
+            float2 sum[NT][KW];
 #pragma unroll
-            for (int t = 0; t < KW; ++t) sum[t] = f2(0.0f);
+            for (int h = 0; h < NT; ++h)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float z[16];
-                tmem_load16(z, tmem + ((uint32_t)warp << 21) + 16 * h);
+                for (int t = 0; t < KW; ++t) sum[h][t] = f2(0.0f);
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                float z[NT][16];
+#pragma unroll
+                for (int h = 0; h < NT; ++h) tmem_load16(z[h], tmem + ((uint32_t)warp << 21) + 32 * h + 16 * half);
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    const float4 *p = reinterpret_cast<const float4 *>(s.w.w3[h * 8 + c]);
+                    const float4 *p = reinterpret_cast<const float4 *>(s.w.w3[half * 8 + c]);
                     const float4 p0 = p[0], p1 = p[1], p2 = p[2];
-                    const float2 g = gelu2_doubled(__fadd2_rn(make_float2(z[2 * c], z[2 * c + 1]), make_float2(p0.x, p0.y)));
-                    sum[0] = __ffma2_rn(make_float2(p0.z, p0.w), g, sum[0]);
-                    sum[1] = __ffma2_rn(make_float2(p1.x, p1.y), g, sum[1]);
-                    sum[2] = __ffma2_rn(make_float2(p1.z, p1.w), g, sum[2]);
-                    sum[3] = __ffma2_rn(make_float2(p2.x, p2.y), g, sum[3]);
-                    sum[4] = __ffma2_rn(make_float2(p2.z, p2.w), g, sum[4]);
+#pragma unroll
+                    for (int h = 0; h < NT; ++h) {
+                        const float2 g =
+                            gelu2_doubled(__fadd2_rn(make_float2(z[h][2 * c], z[h][2 * c + 1]), make_float2(p0.x, p0.y)));
+                        sum[h][0] = __ffma2_rn(make_float2(p0.z, p0.w), g, sum[h][0]);
+                        sum[h][1] = __ffma2_rn(make_float2(p1.x, p1.y), g, sum[h][1]);
+                        sum[h][2] = __ffma2_rn(make_float2(p1.z, p1.w), g, sum[h][2]);
+                        sum[h][3] = __ffma2_rn(make_float2(p2.x, p2.y), g, sum[h][3]);
+                        sum[h][4] = __ffma2_rn(make_float2(p2.z, p2.w), g, sum[h][4]);
+                    }
                 }
             }
 #pragma unroll
-            for (int t = 0; t < KW; ++t) s.p3[t][tid] = sum[t].x + sum[t].y;
+            for (int h = 0; h < NT; ++h)
+#pragma unroll
+                for (int t = 0; t < KW; ++t) s.p3[h][t][tid] = sum[h][t].x + sum[h][t].y;
         }
         if (__syncthreads_or(!done)) {
             if (tid == 0) *(volatile int *)status = 1;
@@ -261,21 +307,22 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
             break;
         }
         parity ^= 1;
-        const uint32_t dom = tile / tiles_per_dom;
-        const int64_t x = (int64_t)(tile - dom * tiles_per_dom) * n_out + tid;
-        if (tid < n_out && x < n) {
-            float d = 0.0f;
 #pragma unroll
-            for (int t = 0; t < KW; ++t) d += s.p3[t][(tid + t) & 127];
-            d = s.w.scale * (d + s.w.b3);
-            out[(int64_t)dom * n + x] = STEP ? v + d : d;
+        for (int h = 0; h < NT; ++h) {
+            if (tid < n_out && at[h] < n) {
+                float d = 0.0f;
+#pragma unroll
+                for (int t = 0; t < KW; ++t) d += s.p3[h][t][(tid + t) & 127];
+                d = s.w.scale * (d + s.w.b3);
+                out[row[h] + at[h]] = STEP ? v[h] + d : d;
+            }
         }
     }
     tcgen05_before_sync();
     __syncthreads();
     if (warp == 0) {
         tcgen05_after_sync();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(FWD_TMEM));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
     }
 }
 
