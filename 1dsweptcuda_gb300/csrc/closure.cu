@@ -87,7 +87,6 @@ namespace cl {
 __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 lo, __nv_bfloat16 hi) {
     return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
-__device__ __forceinline__ uint32_t ld2(const __nv_bfloat16 *p) { return *reinterpret_cast<const uint32_t *>(p); }
 
 // D = A * B + D, m16n8k16, A row-major BF16, B column-major BF16, FP32 accumulate
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -99,37 +98,61 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Four (two) 8 x 8 BF16 matrices into fragments, lane l giving the address of row l % 8 of matrix l / 8; T: transposed.
+template <bool T>
+__device__ __forceinline__ void ldm4(uint32_t (&r)[4], const __nv_bfloat16 *row) {
+    if constexpr (T)
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(smem_addr(row))
+                     : "memory");
+    else
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(smem_addr(row))
+                     : "memory");
+}
+__device__ __forceinline__ void ldm2_t(uint32_t (&r)[2], const __nv_bfloat16 *row) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+                 : "=r"(r[0]), "=r"(r[1])
+                 : "r"(smem_addr(row))
+                 : "memory");
+}
+
 // Shared memory of a tile.
+constexpr int LDT = NZ2 + 8;  // dzT's row stride: 304 bytes, conflict-free fragment reads
 struct Smem {
-    float us[NU];
-    float w1[CH * KW], b1[CH], b2[CH], w3[CH * KW], b3, scale;
-    __nv_bfloat16 a1[NA1 * LDB];                   // layer-1 activations, BF16 (the MMA A operand)
-    alignas(16) __nv_bfloat16 w2[KW * CH * LDB];   // w2[t][o][i], i contiguous (the MMA B operand)
-    float a2[NA2 * LDF];                           // layer-2 activations gelu(z2)
-    float z2[NA2 * LDF];                           // layer-2 pre-activations
-    float z1[NA1 * LDF];                           // layer-1 pre-activations
+    alignas(16) __nv_bfloat16 a1[NA1 * LDB];     // layer-1 activations (an MMA operand)
+    alignas(16) __nv_bfloat16 w2[KW * CH * LDB]; // w2[t][o][i], i contiguous (an MMA operand)
+    alignas(16) __nv_bfloat16 dzT[CH * LDT];     // dz2 as [o][p], p contiguous, for dW2
+    alignas(16) __nv_bfloat16 dzP[LDT * LDB];    // dz2 as [4 + p][o], 4 zero rows in front, for da1
+    alignas(16) float w3[KW * CH];               // [t][i]
+    float w1[CH * KW], b1[CH], b2[CH];
+    float us[NU + 8];                            // the last 8 pad the last warp's window
+    float dd[4 + LDT + 8];                       // dL/ddelta of output q at 4 + q, zeros around it
+    float part[2][TOUT];                         // layer 3: the two channel halves' sums
+    float a2[NA2 * LDF];                         // layer-2 activations gelu(z2)
+    float z2[NA2 * LDF];                         // layer-2 pre-activations
+    float z1[NA1 * LDF];                         // layer-1 pre-activations, then dz1
 };
 
-// Load the tile's inputs (periodic within the domain) and the weights.
-__device__ void load_tile(Smem &s, const float *__restrict__ theta, const float *__restrict__ u, int64_t n,
-                          int64_t x0) {
+// The tile's inputs (periodic within the domain).
+__device__ void load_tile(Smem &s, const float *__restrict__ u, int64_t n, int64_t x0) {
     for (int j = threadIdx.x; j < NU; j += blockDim.x) {
         int64_t q = x0 - 6 + j;
         q %= n;
         if (q < 0) q += n;
         s.us[j] = u[q];
     }
-    for (int i = threadIdx.x; i < CH * KW; i += blockDim.x) {
-        s.w1[i] = bf16r(theta[OW1 + i]);
-        s.w3[i] = bf16r(theta[OW3 + i]);
+}
+__device__ void load_weights(Smem &s, const float *__restrict__ theta) {
+    for (int k = threadIdx.x; k < CH * KW; k += blockDim.x) {
+        s.w1[k] = bf16r(theta[OW1 + k]);
+        s.w3[(k % KW) * CH + k / KW] = bf16r(theta[OW3 + k]);
     }
     for (int i = threadIdx.x; i < CH; i += blockDim.x) {
         s.b1[i] = theta[OB1 + i];
         s.b2[i] = theta[OB2 + i];
-    }
-    if (threadIdx.x == 0) {
-        s.b3 = theta[OB3];
-        s.scale = theta[OSCALE];
     }
     // w2 flat is [o][i][t]; smem is [t][o][i]
     for (int k = threadIdx.x; k < CH * CH * KW; k += blockDim.x) {
@@ -178,172 +201,164 @@ __device__ void forward_12(Smem &s) {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 // rows beyond NA1 are only reached for p >= NA2 (discarded rows): clamp the read
-                const int ra = min(p0 + g + t, NA1 - 1), rb = min(p0 + g + 8 + t, NA1 - 1);
-                const uint32_t a0 = ld2(&s.a1[ra * LDB + 16 * h + 2 * q]);
-                const uint32_t a1 = ld2(&s.a1[rb * LDB + 16 * h + 2 * q]);
-                const uint32_t a2 = ld2(&s.a1[ra * LDB + 16 * h + 8 + 2 * q]);
-                const uint32_t a3 = ld2(&s.a1[rb * LDB + 16 * h + 8 + 2 * q]);
+                uint32_t a[4], b[4];
+                ldm4<false>(a, &s.a1[min(p0 + t + (lane & 15), NA1 - 1) * LDB + 16 * h + (lane >> 4) * 8]);
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) {
-                    const __nv_bfloat16 *wb = &s.w2[(t * CH + nt * 8 + g) * LDB + 16 * h];
-                    mma_bf16(acc[nt], a0, a1, a2, a3, ld2(wb + 2 * q), ld2(wb + 8 + 2 * q));
+                for (int nt = 0; nt < 4; nt += 2) {
+                    ldm4<false>(b, &s.w2[(t * CH + (nt + (lane >> 4)) * 8 + (lane & 7)) * LDB + 16 * h + ((lane >> 3) & 1) * 8]);
+                    mma_bf16(acc[nt], a[0], a[1], a[2], a[3], b[0], b[1]);
+                    mma_bf16(acc[nt + 1], a[0], a[1], a[2], a[3], b[2], b[3]);
                 }
             }
         }
         const int r0 = p0 + g, r1 = p0 + g + 8;
-        {
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) {
-                const int o = nt * 8 + 2 * q;
-                if (r0 < NA2) {
-                    const float z0 = acc[nt][0] + s.b2[o], z1 = acc[nt][1] + s.b2[o + 1];
-                    s.z2[r0 * LDF + o] = z0;
-                    s.z2[r0 * LDF + o + 1] = z1;
-                    s.a2[r0 * LDF + o] = gelu(z0);
-                    s.a2[r0 * LDF + o + 1] = gelu(z1);
-                }
-                if (r1 < NA2) {
-                    const float z2 = acc[nt][2] + s.b2[o], z3 = acc[nt][3] + s.b2[o + 1];
-                    s.z2[r1 * LDF + o] = z2;
-                    s.z2[r1 * LDF + o + 1] = z3;
-                    s.a2[r1 * LDF + o] = gelu(z2);
-                    s.a2[r1 * LDF + o + 1] = gelu(z3);
-                }
+        for (int nt = 0; nt < 4; ++nt) {
+            const int o = nt * 8 + 2 * q;
+            if (r0 < NA2) {
+                const float z0 = acc[nt][0] + s.b2[o], z1 = acc[nt][1] + s.b2[o + 1];
+                s.z2[r0 * LDF + o] = z0;
+                s.z2[r0 * LDF + o + 1] = z1;
+                s.a2[r0 * LDF + o] = gelu(z0);
+                s.a2[r0 * LDF + o + 1] = gelu(z1);
+            }
+            if (r1 < NA2) {
+                const float z2 = acc[nt][2] + s.b2[o], z3 = acc[nt][3] + s.b2[o + 1];
+                s.z2[r1 * LDF + o] = z2;
+                s.z2[r1 * LDF + o + 1] = z3;
+                s.a2[r1 * LDF + o] = gelu(z2);
+                s.a2[r1 * LDF + o + 1] = gelu(z3);
             }
         }
     }
     __syncthreads();
 }
 
-// Layer 3 for output q: b3 + sum_{t,i} w3[i][t] * a2[q + t][i].
-__device__ __forceinline__ float layer3(const Smem &s, int q) {
-    float d = 0.0f;
-#pragma unroll
-    for (int t = 0; t < KW; ++t)
-#pragma unroll 8
-        for (int i = 0; i < CH; ++i) d = fmaf(s.w3[i * KW + t], s.a2[(q + t) * LDF + i], d);
-    return d + s.b3;
-}
-
-// ---------------------------------------------------------------- kernels
 // Loss and parameter gradients (forward + backward), summed over the tiles a
 // block visits into its row of `partial` ([gridDim.x][NPARAM + 1], last = loss).
 // The loss is on the scaled defect: L = wpt * sum (net(u) - target / s)^2,
 // wpt = 1 / (points in the batch), s the output scale.
-__global__ void __launch_bounds__(THREADS) k_grad(const float *__restrict__ theta, const float *__restrict__ u,
-                                                  const float *__restrict__ target, const int64_t *__restrict__ rows,
-                                                  float *__restrict__ partial, int64_t n, int64_t tiles_per_dom,
-                                                  int64_t n_tiles, float scale) {
+//
+// Bound by latency: a tile is a chain of eight short phases, 512 tiles (a minibatch
+// of 64 x 1024) on 152 SMs.  So the small layers' sums run with a lane per channel,
+// each warp on its own rows with a sliding window, and stay in registers from tile
+// to tile (sums over all rows by a few threads, through shared memory, took half of
+// the tile); fragments are loaded with ldmatrix, transposed where the operand lies
+// the other way; and a block's 100 KB of shared memory lets two share an SM.
+__global__ void __launch_bounds__(THREADS, 2) k_grad(const float *__restrict__ theta, const float *__restrict__ u,
+                                                     const float *__restrict__ target, const int64_t *__restrict__ rows,
+                                                     float *__restrict__ partial, int64_t n, int64_t tiles_per_dom,
+                                                     int64_t n_tiles, float scale) {
     extern __shared__ __align__(16) unsigned char raw[];
     Smem &s = *reinterpret_cast<Smem *>(raw);
-    __shared__ float g[NPARAM + 1];                 // this block's sums of the small-layer gradients and the loss
-    __shared__ float dd[TOUT];                      // dL/ddelta
-    __shared__ __nv_bfloat16 dzT[CH * (NZ2 + 8)];   // dz2 as [o][p] (BF16), p contiguous, for dW2
-    __shared__ __nv_bfloat16 dzP[(NZ2 + 8) * LDB];  // dz2 as [4 + p][o] (BF16), 4 zero rows in front, for da1
-    for (int i = threadIdx.x; i < NPARAM + 1; i += blockDim.x) g[i] = 0.0f;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, q4 = lane & 3;
-    const int nwarp = blockDim.x >> 5;
-    // dW2 accumulators: warp w owns (m-tile mo, n-tile nn) pairs k = w, w+8, ... of 2 x 20
-    float accw[5][4] = {};
+    constexpr int NW = THREADS / 32;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, gq = lane >> 2, q4 = lane & 3;
+    load_weights(s, theta);
+    for (int i = tid; i < 4 + LDT + 8; i += THREADS) s.dd[i] = 0.0f;
+    if (tid < 8) s.us[NU + tid] = 0.0f;
+    for (int i = tid; i < 4 * LDB; i += THREADS) s.dzP[i] = __float2bfloat16_rn(0.0f);
+    const float b3 = theta[OB3], out_scale = theta[OSCALE];
     __syncthreads();
+    float w3[KW];  // channel `lane`
+#pragma unroll
+    for (int t = 0; t < KW; ++t) w3[t] = s.w3[t * CH + lane];
+    // this thread's sums: dW2 of output channels 16 (warp / 4) on and columns (t, i) of n-tiles 5 (warp % 4) on;
+    // channel `lane`'s dW1, db1, dW3, db2 over its warp's rows; db3 and the loss over its outputs
+    float accw[5][4] = {}, dw1[KW] = {}, dw3[KW] = {}, db1 = 0.0f, db2 = 0.0f, db3 = 0.0f, loss = 0.0f;
 
     for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const int64_t b = tile / tiles_per_dom, x0 = (tile % tiles_per_dom) * TOUT;
         const int64_t dom = rows ? rows[b] : b;  // minibatch row -> sample
-        load_tile(s, theta, u + dom * n, n, x0);
+        load_tile(s, u + dom * n, n, x0);
+        const float want = tid < TOUT ? target[dom * n + x0 + tid] : 0.0f;
         __syncthreads();
         forward_12(s);
-        // delta, dL/ddelta, loss, dW3, db3
-        for (int q = threadIdx.x; q < TOUT; q += blockDim.x) {
-            const float d = layer3(s, q);
-            const float e = d - target[dom * n + x0 + q] / s.scale;
-            dd[q] = 2.0f * scale * e;
-            atomicAdd(&g[NPARAM], scale * e * e);
-        }
-        __syncthreads();
-        for (int k = threadIdx.x; k < CH * KW; k += blockDim.x) {
-            const int i = k / KW, t = k % KW;
-            float a = 0.0f;
-            for (int q = 0; q < TOUT; ++q) a = fmaf(dd[q], s.a2[(q + t) * LDF + i], a);
-            g[OW3 + k] += a;
-        }
-        if (threadIdx.x < 32) {
-            float a = 0.0f;
-            for (int q = threadIdx.x; q < TOUT; q += 32) a += dd[q];
+        {  // layer 3, half of the channels per thread
+            const int q = tid & (TOUT - 1), i0 = (tid / TOUT) * (CH / 2);
+            float d = 0.0f;
 #pragma unroll
-            for (int off = 16; off; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
-            if (threadIdx.x == 0) g[OB3] += a;
-        }
-        // dz2[p][o] = (sum_t w3[o][t] dd[p - t]) * gelu'(z2[p][o]), p < NA2; zero beyond
-        for (int k = threadIdx.x; k < (NZ2 + 8) * CH; k += blockDim.x) {
-            const int p = k / CH, o = k % CH;
-            float v = 0.0f;
-            if (p < NA2) {
-                float da = 0.0f;
+            for (int t = 0; t < KW; ++t)
 #pragma unroll
-                for (int t = 0; t < KW; ++t) {
-                    const int qq = p - t;
-                    if (qq >= 0 && qq < TOUT) da = fmaf(s.w3[o * KW + t], dd[qq], da);
+                for (int i = 0; i < CH / 2; i += 4) {
+                    const float4 w = *reinterpret_cast<const float4 *>(&s.w3[t * CH + i0 + i]);
+                    const float *a = &s.a2[(q + t) * LDF + i0 + i];
+                    d = fmaf(w.x, a[0], d);
+                    d = fmaf(w.y, a[1], d);
+                    d = fmaf(w.z, a[2], d);
+                    d = fmaf(w.w, a[3], d);
                 }
-                v = da * gelu_grad(s.z2[p * LDF + o]);
-            }
-            const __nv_bfloat16 b = __float2bfloat16_rn(v);
-            dzT[o * (NZ2 + 8) + p] = b;
-            if (p + 4 < NZ2 + 8) dzP[(p + 4) * LDB + o] = b;
-            if (p < 4) dzP[p * LDB + o] = __float2bfloat16_rn(0.0f);
+            s.part[tid / TOUT][q] = d;
         }
         __syncthreads();
-        // db2
-        for (int o = threadIdx.x; o < CH; o += blockDim.x) {
-            float a = 0.0f;
-            for (int p = 0; p < NA2; ++p) a += __bfloat162float(dzT[o * (NZ2 + 8) + p]);
-            g[OB2 + o] += a;
+        if (tid < TOUT) {
+            const float e = (s.part[0][tid] + s.part[1][tid] + b3) - want / out_scale;
+            const float g = 2.0f * scale * e;
+            s.dd[4 + tid] = g;
+            loss += scale * e * e;
+            db3 += g;
         }
-        // dW2[o][(t,i)] += sum_p dz2[p][o] a1[p + t][i]: M = o (2 tiles), N = (t, i) (20 tiles), K = p (9 steps)
+        __syncthreads();
+        {  // dz2[p][o] = (sum_t w3[o][t] dd[p - t]) * gelu'(z2[p][o]), p < NA2, zero beyond; dW3, db2
+            constexpr int PER = 20;  // rows per warp (even: they are stored in pairs)
+            const int p0 = warp * PER, p1 = min(p0 + PER, LDT);
+            float w[KW];  // w[t] = dd[p - t]
 #pragma unroll
-        for (int slot = 0; slot < 5; ++slot) {
-            const int k = warp + slot * 8;  // 8 warps x 5 slots = 40 (m-tile, n-tile) pairs
-            const int mo = k / 20, nn = k % 20, t = nn / 4, i0 = (nn % 4) * 8;
-            for (int ks = 0; ks < NZ2 / 16; ++ks) {
-                const int p0 = ks * 16;
-                const __nv_bfloat16 *ra = &dzT[(mo * 16 + gq) * (NZ2 + 8) + p0];
-                const __nv_bfloat16 *rb = &dzT[(mo * 16 + gq + 8) * (NZ2 + 8) + p0];
-                const uint32_t a0 = ld2(ra + 2 * q4), a1 = ld2(rb + 2 * q4);
-                const uint32_t a2 = ld2(ra + 8 + 2 * q4), a3 = ld2(rb + 8 + 2 * q4);
-                // B[k = p][n = i]: a1[p0 + k + t][i0 + gq]; rows past NA1 meet dz2 = 0
-                const int c = i0 + gq;
-                const int r0 = min(p0 + 2 * q4 + t, NA1 - 1), r1 = min(p0 + 2 * q4 + 1 + t, NA1 - 1);
-                const int r2 = min(p0 + 8 + 2 * q4 + t, NA1 - 1), r3 = min(p0 + 9 + 2 * q4 + t, NA1 - 1);
-                const uint32_t b0 = pack2(s.a1[r0 * LDB + c], s.a1[r1 * LDB + c]);
-                const uint32_t b1 = pack2(s.a1[r2 * LDB + c], s.a1[r3 * LDB + c]);
-                mma_bf16(accw[slot], a0, a1, a2, a3, b0, b1);
+            for (int t = 0; t < KW - 1; ++t) w[t] = s.dd[p0 + 3 - t];
+            for (int p = p0; p < p1; p += 2) {
+                __nv_bfloat16 z[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+#pragma unroll
+                    for (int t = KW - 1; t > 0; --t) w[t] = w[t - 1];
+                    w[0] = s.dd[p + k + 4];
+                    float v = 0.0f;
+                    if (p + k < NA2) {
+                        float da = 0.0f;
+                        const float a = s.a2[(p + k) * LDF + lane];
+#pragma unroll
+                        for (int t = 0; t < KW; ++t) {
+                            da = fmaf(w3[t], w[t], da);
+                            dw3[t] = fmaf(w[t], a, dw3[t]);
+                        }
+                        v = da * gelu_grad(s.z2[(p + k) * LDF + lane]);
+                    }
+                    z[k] = __float2bfloat16_rn(v);
+                    db2 += __bfloat162float(z[k]);
+                    if (p + k + 4 < LDT) s.dzP[(p + k + 4) * LDB + lane] = z[k];
+                }
+                *reinterpret_cast<uint32_t *>(&s.dzT[lane * LDT + p]) = pack2(z[0], z[1]);
+            }
+        }
+        __syncthreads();
+        // dW2[o][(t,i)] += sum_p dz2[p][o] a1[p + t][i]: M = o (2 tiles), N = (t, i) (20 tiles), K = p (9 steps);
+        // rows past NA1 meet dz2 = 0
+        for (int ks = 0; ks < NZ2 / 16; ++ks) {
+            uint32_t a[4], f[2];
+            ldm4<false>(a, &s.dzT[((warp >> 2) * 16 + (lane & 15)) * LDT + ks * 16 + (lane >> 4) * 8]);
+#pragma unroll
+            for (int slot = 0; slot < 5; ++slot) {
+                const int nn = (warp & 3) * 5 + slot, t = nn / 4, i0 = (nn % 4) * 8;
+                ldm2_t(f, &s.a1[min(ks * 16 + t + (lane & 15), NA1 - 1) * LDB + i0]);
+                mma_bf16(accw[slot], a[0], a[1], a[2], a[3], f[0], f[1]);
             }
         }
         // da1[r][i] = sum_{t,o} w2[o][i][t] dz2[r - t][o]: M = r (10 tiles of 16 over NA1), N = i (4), K = (t, o) (10)
-        // then dz1 = da1 * gelu'(z1), db1, dW1
-        for (int m = warp; m < (NA1 + 15) / 16; m += nwarp) {
+        // then dz1 = da1 * gelu'(z1)
+        for (int m = warp; m < (NA1 + 15) / 16; m += NW) {
             const int r0 = m * 16;
             float acc[4][4] = {};
 #pragma unroll
             for (int t = 0; t < KW; ++t) {
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    // A[r][o] = dz2[r - t][o] = dzP[(r - t + 4)][o]; rows beyond the buffer are zero-padded
-                    const int ra = min(r0 + gq - t + 4, NZ2 + 7), rb = min(r0 + gq + 8 - t + 4, NZ2 + 7);
-                    const uint32_t a0 = ld2(&dzP[ra * LDB + 16 * h + 2 * q4]);
-                    const uint32_t a1 = ld2(&dzP[rb * LDB + 16 * h + 2 * q4]);
-                    const uint32_t a2 = ld2(&dzP[ra * LDB + 16 * h + 8 + 2 * q4]);
-                    const uint32_t a3 = ld2(&dzP[rb * LDB + 16 * h + 8 + 2 * q4]);
+                    // A[r][o] = dz2[r - t][o] = dzP[r - t + 4][o]; rows beyond NA1 are discarded: clamp the read
+                    uint32_t a[4], f[4];
+                    ldm4<false>(a, &s.dzP[min(r0 + (lane & 15) - t + 4, LDT - 1) * LDB + 16 * h + (lane >> 4) * 8]);
 #pragma unroll
-                    for (int nt = 0; nt < 4; ++nt) {
-                        // B[k = o][n = i] = w2[o][i][t]: column i contiguous over o is w2[t] transposed;
-                        // w2 smem is [t][o][i], so gather the two o values of the pair
-                        const int ic = nt * 8 + gq;
-                        const int o0 = 16 * h + 2 * q4;
-                        const uint32_t b0 = pack2(s.w2[(t * CH + o0) * LDB + ic], s.w2[(t * CH + o0 + 1) * LDB + ic]);
-                        const uint32_t b1 =
-                            pack2(s.w2[(t * CH + o0 + 8) * LDB + ic], s.w2[(t * CH + o0 + 9) * LDB + ic]);
-                        mma_bf16(acc[nt], a0, a1, a2, a3, b0, b1);
+                    for (int nt = 0; nt < 4; nt += 2) {
+                        ldm4<true>(f, &s.w2[(t * CH + 16 * h + (lane & 15)) * LDB + (nt + (lane >> 4)) * 8]);
+                        mma_bf16(acc[nt], a[0], a[1], a[2], a[3], f[0], f[1]);
+                        mma_bf16(acc[nt + 1], a[0], a[1], a[2], a[3], f[2], f[3]);
                     }
                 }
             }
@@ -357,41 +372,83 @@ __global__ void __launch_bounds__(THREADS) k_grad(const float *__restrict__ thet
             }
         }
         __syncthreads();
-        for (int k = threadIdx.x; k < CH * (KW + 1); k += blockDim.x) {
-            const int o = k / (KW + 1), t = k % (KW + 1);
-            float a = 0.0f;
-            if (t < KW) {
-                for (int r = 0; r < NA1; ++r) a = fmaf(s.z1[r * LDF + o], s.us[r + t], a);
-                g[OW1 + o * KW + t] += a;
-            } else {
-                for (int r = 0; r < NA1; ++r) a += s.z1[r * LDF + o];
-                g[OB1 + o] += a;
+        {  // dW1, db1
+            constexpr int PER = (NA1 + NW - 1) / NW;
+            const int r0 = warp * PER, r1 = min(r0 + PER, NA1);
+            float w[KW];  // w[t] = us[r + t]
+#pragma unroll
+            for (int t = 0; t < KW - 1; ++t) w[t + 1] = s.us[r0 + t];
+            for (int r = r0; r < r1; ++r) {
+#pragma unroll
+                for (int t = 0; t < KW - 1; ++t) w[t] = w[t + 1];
+                w[KW - 1] = s.us[r + KW - 1];
+                const float z = s.z1[r * LDF + lane];
+#pragma unroll
+                for (int t = 0; t < KW; ++t) dw1[t] = fmaf(z, w[t], dw1[t]);
+                db1 += z;
             }
         }
         __syncthreads();
     }
-    // dW2 accumulators -> g (flat w2 is [o][i][t])
+    float *row = partial + (int64_t)blockIdx.x * (NPARAM + 1);
+    // dW2 (flat w2 is [o][i][t])
 #pragma unroll
     for (int slot = 0; slot < 5; ++slot) {
-        const int k = warp + slot * 8;
-        const int mo = k / 20, nn = k % 20, t = nn / 4, i0 = (nn % 4) * 8;
+        const int nn = (warp & 3) * 5 + slot, t = nn / 4, i0 = (nn % 4) * 8;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-            const int o = mo * 16 + gq + (e >= 2 ? 8 : 0), i = i0 + 2 * q4 + (e & 1);
-            g[OW2 + (o * CH + i) * KW + t] += accw[slot][e];
+            const int o = (warp >> 2) * 16 + gq + (e >= 2 ? 8 : 0), i = i0 + 2 * q4 + (e & 1);
+            row[OW2 + (o * CH + i) * KW + t] = accw[slot][e];
         }
     }
+    // the other sums over the warps: red[value][warp][lane], values dW1 x 5, db1, dW3 x 5, db2, db3, loss
+    constexpr int NV = 2 * (KW + 1) + 2;
+    static_assert(NV * THREADS <= NA1 * LDF, "the reduction takes z1's place");
+    float *red = s.z1;
+#pragma unroll
+    for (int t = 0; t < KW; ++t) {
+        red[t * THREADS + tid] = dw1[t];
+        red[(KW + 1 + t) * THREADS + tid] = dw3[t];
+    }
+    red[KW * THREADS + tid] = db1;
+    red[(2 * KW + 1) * THREADS + tid] = db2;
+    red[(2 * KW + 2) * THREADS + tid] = db3;
+    red[(2 * KW + 3) * THREADS + tid] = loss;
     __syncthreads();
-    float *row = partial + (int64_t)blockIdx.x * (NPARAM + 1);
-    for (int i = threadIdx.x; i < NPARAM + 1; i += blockDim.x) row[i] = g[i];
+    for (int v = warp; v < NV; v += NW) {
+        float a = 0.0f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) a += red[v * THREADS + w * 32 + lane];
+        if (v >= 2 * (KW + 1)) {
+#pragma unroll
+            for (int off = 16; off; off >>= 1) a += __shfl_xor_sync(0xffffffffu, a, off);
+            if (lane == 0) row[v == 2 * (KW + 1) ? OB3 : NPARAM] = a;
+        } else {
+            const int t = v % (KW + 1);
+            row[v <= KW ? (t < KW ? OW1 + lane * KW + t : OB1 + lane) : (t < KW ? OW3 + lane * KW + t : OB2 + lane)] = a;
+        }
+    }
+    if (tid == 0) row[OSCALE] = 0.0f;  // not trained
 }
 
-// Sum the blocks' rows: out[j] = sum_b partial[b][j], j < NPARAM + 1.
-__global__ void k_reduce(const float *__restrict__ partial, int rows, float *__restrict__ out) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= NPARAM + 1) return;
+// Sum the blocks' rows: out[j] = sum_b partial[b][j], j < NPARAM + 1.  A block takes 32 values, each warp every eighth
+// row (one thread per value, 304 rows in a chain, took 16 us).
+constexpr int REDUCE_WARPS = 8;
+__global__ void __launch_bounds__(32 * REDUCE_WARPS) k_reduce(const float *__restrict__ partial, int rows,
+                                                              float *__restrict__ out) {
+    __shared__ float sums[REDUCE_WARPS][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = blockIdx.x * 32 + lane;
     float a = 0.0f;
-    for (int b = 0; b < rows; ++b) a += partial[(int64_t)b * (NPARAM + 1) + j];
+    if (j < NPARAM + 1) {
+#pragma unroll 8
+        for (int b = warp; b < rows; b += REDUCE_WARPS) a += partial[(int64_t)b * (NPARAM + 1) + j];
+    }
+    sums[warp][lane] = a;
+    __syncthreads();
+    if (warp || j >= NPARAM + 1) return;
+    a = 0.0f;
+#pragma unroll
+    for (int w = 0; w < REDUCE_WARPS; ++w) a += sums[w][lane];
     out[j] = a;
 }
 
@@ -636,7 +693,7 @@ int sw_closure_grad(sw_ctx *ctx, const float *theta, const float *u, const float
     cl::k_grad<<<(unsigned)grid, cl::THREADS, cl::smem_bytes(), ctx->stream>>>(theta, u, target, rows, partial, n,
                                                                                 tiles_per, n_tiles, scale);
     SW_CUDA(ctx, cudaGetLastError());
-    cl::k_reduce<<<(cl::NPARAM + 1 + 255) / 256, 256, 0, ctx->stream>>>(partial, (int)grid, grad_and_loss);
+    cl::k_reduce<<<(cl::NPARAM + 1 + 31) / 32, 32 * cl::REDUCE_WARPS, 0, ctx->stream>>>(partial, (int)grid, grad_and_loss);
     SW_CUDA(ctx, cudaGetLastError());
     SW_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return SW_OK;
