@@ -38,7 +38,7 @@ NVCC_FLAGS += os.environ.get("SW_NVCC_EXTRA", "").split()
 CU_SOURCES = ["k_heat.cu", "k_ks.cu", "k_ks_div.cu", "k_euler.cu", "api.cu", "batch.cu", "noalloc.cu", "closure.cu", "diag.cu",
               "host_tile.cu"]
 CPP_SOURCES = ["cli.cpp"]
-HEADERS = ["engine.cuh", "stencils.cuh", "persistent.cuh", "swept_pair.cuh", "closure_fwd.cuh", "launch.cuh", "sw_internal.h", "ctx.h", "exact_int.h"]
+HEADERS = ["engine.cuh", "stencils.cuh", "persistent.cuh", "swept_pair.cuh", "swept_heat.cuh", "closure_fwd.cuh", "launch.cuh", "sw_internal.h", "ctx.h", "exact_int.h"]
 PROGRAMS = [(p, pi, q, qi) for pi, p in enumerate(("Heat", "KS", "Euler")) for q, qi in (("Single", 4), ("Double", 8))]
 
 
