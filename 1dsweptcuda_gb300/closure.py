@@ -393,7 +393,7 @@ def bench_target(solver) -> dict:
 
 
 def bench_step(n_dom: int = 1024, steps: int = 200, seed: int = 0, solver=None, closure=None) -> dict:
-    """Throughput of the fused coarse step with the closure on (k_step) and
+    """Throughput of the fused coarse step with the closure on (k_forward) and
     off, on n_dom domains of the coarse grid from a smooth state: ms per step
     of the whole ensemble, coarse cell-steps per second and the tensor-core
     work implied (the 32 -> 32 layer is 2 * 32 * 32 * 5 FLOP per cell)."""

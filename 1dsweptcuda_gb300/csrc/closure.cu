@@ -3,9 +3,8 @@
 // Parameters are FP32 masters rounded to BF16 for the forward pass.  The
 // 32 -> 32 layer -- 94 % of the work -- runs on the tensor cores
 // (tcgen05.mma in the forward pass, mma.sync.m16n8k16 in the backward pass; BF16
-// operands, FP32 accumulation);
-// the 1 -> 32 and 32 -> 1 layers run in FP32 on the CUDA cores with the
-// BF16-rounded weights.  oracle/closure.py restates the same arithmetic.
+// operands, FP32 accumulation); the 1 -> 32 and 32 -> 1 layers run in FP32 on the
+// CUDA cores with the BF16-rounded weights.  oracle/closure.py restates the same arithmetic.
 //
 // The forward pass alone (inference, the coarse step) is closure_fwd.cuh; this
 // file has the backward pass, training and the certified adaptive run.
@@ -46,7 +45,7 @@ constexpr int NZ2 = 144;        // 9 m-tiles of 16 rows
 constexpr int NA2 = TOUT + 4;   // 132 a2 rows used
 constexpr int LDB = 40;         // bf16 row stride (80 B: conflict-free fragment reads)
 constexpr int LDF = 33;         // fp32 row stride
-constexpr int THREADS = 256;  // (9 warps, one per layer-2 m-tile, measured slower: 106.5 against 102.3 us per step)
+constexpr int THREADS = 256;
 // parameter offsets (flat FP32 vector); the last value is the output scale s
 // (delta = s * net(u)), fixed by the caller and left alone by training
 constexpr int OW1 = 0, OB1 = 160, OW2 = 192, OB2 = 5312, OW3 = 5344, OB3 = 5504, OSCALE = 5505;
