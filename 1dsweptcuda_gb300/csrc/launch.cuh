@@ -16,7 +16,8 @@ namespace sw {
 __device__ __forceinline__ void wait_for_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // A launch that may be scheduled while the launch before it drains
-// (wait_for_previous_launch).
+// (wait_for_previous_launch).  Its error is returned and not left behind as the
+// thread's last one, which the end of the next run would report again.
 template <typename... K, typename... A>
 cudaError_t launch_dependent(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchConfig_t cfg = {};
@@ -29,7 +30,9 @@ cudaError_t launch_dependent(void (*kernel)(K...), unsigned grid, unsigned block
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, K(args)...);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 }  // namespace sw
