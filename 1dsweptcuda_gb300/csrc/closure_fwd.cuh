@@ -133,9 +133,8 @@ __device__ __forceinline__ bool umma_wait(uint64_t *bar, unsigned parity) {
 // *status (pinned host memory).
 template <bool STEP, int NT>
 __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
-    k_forward(const FwdWeights *__restrict__ weights, const Params<float> pk, const float *__restrict__ u,
-              float *__restrict__ out, const int64_t n, const uint32_t tiles_per_dom, const uint32_t n_tiles,
-              const int n_out, int *status) {
+    k_forward(const FwdWeights *__restrict__ weights, const Params<float> pk, const float *u, float *out,
+              const int64_t n, const uint32_t tiles_per_dom, const uint32_t n_tiles, const int n_out, int *status) {
     __shared__ FwdSmem<NT> s;
     constexpr uint32_t TMEM_COLS = 32 * NT;  // the blocks that fit an SM's shared memory use at most 384 of its 512
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -330,8 +329,8 @@ __global__ void __launch_bounds__(FWD_THREADS, FWD_BLOCKS)
 // cells need from 12 values (neighbouring lanes share them through L1): no barriers, no shared memory.
 constexpr int PLAIN_THREADS = 256;
 __global__ void __launch_bounds__(PLAIN_THREADS)
-    k_plain_step(const Params<float> pk, const float *__restrict__ u, float *__restrict__ out, const int64_t n,
-                 const uint32_t warps_per_dom, const uint32_t n_warps) {
+    k_plain_step(const Params<float> pk, const float *u, float *out, const int64_t n, const uint32_t warps_per_dom,
+                 const uint32_t n_warps) {
     wait_for_previous_launch();
     const uint32_t wid = blockIdx.x * (PLAIN_THREADS / 32) + (threadIdx.x >> 5);
     if (wid >= n_warps) return;

@@ -689,9 +689,9 @@ inline int swept_threads_for(int W, int threads) {
 // up-triangle -> slots (phase 0 only).  MODE_DIAMOND: slots -> down + up ->
 // slots.  MODE_DOWN: slots -> down-triangle -> state.
 template <int P, typename T, int MODE, int PATH = PATH_ANY>
-__device__ __forceinline__ void swept_tile(const Params<T> &p, typename Scheme<P, T>::G *__restrict__ state,
-                                           typename Scheme<P, T>::G *__restrict__ slots, T *rows, const int W,
-                                           const int phase, const int64_t t) {
+__device__ __forceinline__ void swept_tile(const Params<T> &p, typename Scheme<P, T>::G *state,
+                                           typename Scheme<P, T>::G *slots, T *rows, const int W, const int phase,
+                                           const int64_t t) {
     const int L = row_stride(W), h = W >> 1;
     const int64_t nx = p.nx, nhalf = nx / h;
     const int64_t base = t * W + (int64_t)phase * h;
@@ -732,9 +732,8 @@ constexpr int swept_min_blocks() {
 }
 template <int P, typename T, int MODE, int PATH>
 __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PATH>()))
-    k_swept(const Params<T> p, typename Scheme<P, T>::G *__restrict__ state,
-                                                typename Scheme<P, T>::G *__restrict__ slots, const int W,
-                                                const int phase) {
+    k_swept(const Params<T> p, typename Scheme<P, T>::G *state, typename Scheme<P, T>::G *slots, const int W,
+            const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     swept_tile<P, T, MODE, PATH>(p, state, slots, reinterpret_cast<T *>(sw_smem), W, phase, (int64_t)blockIdx.x);
@@ -746,8 +745,7 @@ __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PA
 // A KS cell of the classic step on the FP64 pipe alone (a cell whose
 // integer-pipe products were flagged, as in tile_point).
 template <typename T>
-__device__ __noinline__ void classic_ks_pipe(const Params<T> &p, const T *__restrict__ in, T *__restrict__ out,
-                                             const int sub, const int64_t g) {
+__device__ __noinline__ void classic_ks_pipe(const Params<T> &p, const T *in, T *out, const int sub, const int64_t g) {
     const int64_t nx = p.nx;
     T v[5];
 #pragma unroll
@@ -755,14 +753,13 @@ __device__ __noinline__ void classic_ks_pipe(const Params<T> &p, const T *__rest
     out[g] = sub == 0 ? ks_predict(p, v[0], v[1], v[2], v[3], v[4]) : ks_correct(p, out[g], v[0], v[1], v[2], v[3], v[4]);
 }
 template <typename T>
-__device__ __noinline__ void classic_heat_pipe(const Params<T> &p, const T *__restrict__ in, T *__restrict__ out,
-                                               const int64_t l, const int64_t g, const int64_t r) {
+__device__ __noinline__ void classic_heat_pipe(const Params<T> &p, const T *in, T *out, const int64_t l, const int64_t g,
+                                               const int64_t r) {
     out[g] = heat_step(p, in[l], in[g], in[r]);
 }
 template <int P, typename T>
-__device__ __forceinline__ void classic_cell(const Params<T> &p, const typename Scheme<P, T>::G *__restrict__ in,
-                                             typename Scheme<P, T>::G *__restrict__ out, const int sub,
-                                             const int64_t g) {
+__device__ __forceinline__ void classic_cell(const Params<T> &p, const typename Scheme<P, T>::G *in,
+                                             typename Scheme<P, T>::G *out, const int sub, const int64_t g) {
     const int64_t nx = p.nx;
     if constexpr (P == SW_HEAT) {
         int64_t l = g - 1, r = g + 1;
@@ -834,8 +831,8 @@ __device__ __forceinline__ void classic_cell(const Params<T> &p, const typename 
 // above, KS 12.3 -> 5.4 us per sub-step, Heat 12.3 -> 5.0.  Same arithmetic as
 // classic_cell, cell for cell.
 template <int P>
-__device__ __forceinline__ void classic_cells4(const Params<float> &p, const float *__restrict__ in,
-                                               float *__restrict__ out, const int sub, const int64_t x0) {
+__device__ __forceinline__ void classic_cells4(const Params<float> &p, const float *in, float *out, const int sub,
+                                               const int64_t x0) {
     const int64_t nx = p.nx;
     const float4 c = *reinterpret_cast<const float4 *>(in + x0);
     if constexpr (P == SW_HEAT) {
@@ -866,16 +863,15 @@ __device__ __forceinline__ void classic_cells4(const Params<float> &p, const flo
     }
 }
 template <int P>
-__global__ void __launch_bounds__(256) k_classic4(const Params<float> p, const float *__restrict__ in,
-                                                  float *__restrict__ out, const int sub) {
+__global__ void __launch_bounds__(256) k_classic4(const Params<float> p, const float *in, float *out, const int sub) {
     const int64_t x0 = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
     wait_for_previous_launch();
     if (x0 < p.nx) classic_cells4<P>(p, in, out, sub, x0);
 }
 
 template <int P, typename T>
-__global__ void __launch_bounds__(Scheme<P, T>::CMAXT) k_classic(const Params<T> p, const typename Scheme<P, T>::G *__restrict__ in,
-                                                  typename Scheme<P, T>::G *__restrict__ out, const int sub) {
+__global__ void __launch_bounds__(Scheme<P, T>::CMAXT) k_classic(const Params<T> p, const typename Scheme<P, T>::G *in,
+                                                  typename Scheme<P, T>::G *out, const int sub) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     wait_for_previous_launch();
     if (g < p.nx) classic_cell<P, T>(p, in, out, sub, g);
@@ -886,8 +882,8 @@ __global__ void __launch_bounds__(Scheme<P, T>::CMAXT) k_classic(const Params<T>
 // hold the Dirichlet states (classicEuler, Euler1D_SweptShared.cu:400-426).
 // FP64: four blocks per SM (64 registers), 3 % faster than three and 7 % than five.
 template <typename T>
-__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 0) k_classic_euler(const Params<T> p, const V4<T> *__restrict__ in,
-                                                       V4<T> *__restrict__ out, const int sub) {
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 4 : 0) k_classic_euler(const Params<T> p, const V4<T> *in, V4<T> *out,
+                                                                                 const int sub) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t b = warp * kEulerCellsPerWarp + lane, nx = p.nx;
@@ -1076,7 +1072,7 @@ __device__ __forceinline__ void group_bulk_export(T *slots, T *rows, int TS, int
 }
 
 template <int P, typename T, int MODE, int G, int PATH>
-__device__ __forceinline__ void swept_tile_group(const Params<T> &p, T *__restrict__ state, T *__restrict__ slots,
+__device__ __forceinline__ void swept_tile_group(const Params<T> &p, T *state, T *slots,
                                                  T *rows, const int W, const int phase, const int64_t t0) {
     static_assert(P != SW_EULER, "Euler tiles are not grouped");
     constexpr int R = Scheme<P, T>::R;
@@ -1136,8 +1132,7 @@ __device__ __forceinline__ void swept_tile_group(const Params<T> &p, T *__restri
 // Two 1024-thread blocks per SM (32 registers): the FP64 levels need the
 // warps of both to keep the FP64 pipe fed across each level's barrier.
 template <int P, typename T, int MODE, int G, int PATH>
-__global__ void __launch_bounds__(1024, 2) k_swept_group(const Params<T> p, T *__restrict__ state,
-                                                      T *__restrict__ slots, const int W, const int phase) {
+__global__ void __launch_bounds__(1024, 2) k_swept_group(const Params<T> p, T *state, T *slots, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     swept_tile_group<P, T, MODE, G, PATH>(p, state, slots, reinterpret_cast<T *>(sw_smem), W, phase,
@@ -1254,7 +1249,7 @@ __device__ __forceinline__ void ks_warp4_level(const Params<T> &p, int par, int 
 
 template <typename T, int MODE>
 __global__ void __launch_bounds__(32 * kKsWarpTilesPerBlock)
-    k_swept_ks_warp(const Params<T> p, T *__restrict__ state, T *__restrict__ slots, const int phase,
+    k_swept_ks_warp(const Params<T> p, T *state, T *slots, const int phase,
                     const int64_t ntile) {
     constexpr int W = kKsWarpTile, h = W / 2, R = 2, H = W / (2 * R);
     const int lane = threadIdx.x & 31, c0 = 4 * lane;

@@ -299,8 +299,8 @@ cudaError_t launch_persistent_ks_smem_nodes(const Params<T> &p, T *st, T *sl, un
 
 template <int P, typename T, int MODE, int PATH>
 __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PATH>()))
-    k_swept_batch(const Params<T> p, typename Scheme<P, T>::G *__restrict__ state,
-                  typename Scheme<P, T>::G *__restrict__ slots, const BatchDev b, const int W, const int phase) {
+    k_swept_batch(const Params<T> p, typename Scheme<P, T>::G *state, typename Scheme<P, T>::G *slots, const BatchDev b,
+                  const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     const int64_t g = blockIdx.x;
@@ -317,8 +317,7 @@ __global__ void __launch_bounds__(Scheme<P, T>::MAXT, (swept_min_blocks<P, T, PA
 // multiples of G (BatchDev::group), so a block's tiles never straddle domains.
 template <int P, typename T, int MODE, int G, int PATH>
 __global__ void __launch_bounds__(1024, 2)
-    k_swept_batch_group(const Params<T> p, T *__restrict__ state, T *__restrict__ slots, const BatchDev b, const int W,
-                        const int phase) {
+    k_swept_batch_group(const Params<T> p, T *state, T *slots, const BatchDev b, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     wait_for_previous_launch();
     const int64_t g0 = G * (int64_t)blockIdx.x;
@@ -336,8 +335,8 @@ __global__ void __launch_bounds__(1024, 2)
 // block.
 template <int P, typename T>
 __global__ void __launch_bounds__(kClassicBlock)
-    k_classic_batch(const Params<T> p, const typename Scheme<P, T>::G *__restrict__ in,
-                    typename Scheme<P, T>::G *__restrict__ out, const BatchDev b, const int sub) {
+    k_classic_batch(const Params<T> p, const typename Scheme<P, T>::G *in,
+                    typename Scheme<P, T>::G *out, const BatchDev b, const int sub) {
     const int64_t g = (int64_t)blockIdx.x * kClassicBlock + threadIdx.x;
     wait_for_previous_launch();
     if (g >= b.n_cells) return;
@@ -353,8 +352,7 @@ __global__ void __launch_bounds__(kClassicBlock)
 // multiple of 4 (BatchDev::vec4).
 template <int P>
 __global__ void __launch_bounds__(kClassicBlock)
-    k_classic4_batch(const Params<float> p, const float *__restrict__ in, float *__restrict__ out, const BatchDev b,
-                     const int sub) {
+    k_classic4_batch(const Params<float> p, const float *in, float *out, const BatchDev b, const int sub) {
     const int64_t g = 4 * ((int64_t)blockIdx.x * kClassicBlock + threadIdx.x);
     wait_for_previous_launch();
     if (g >= b.n_cells) return;

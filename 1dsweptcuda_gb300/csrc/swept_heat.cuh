@@ -184,7 +184,7 @@ __device__ __forceinline__ void heat_tile_up(const Params<float> &p, float *rows
 constexpr int kHeatMaxTile = 1024;
 template <int MODE>
 __global__ void __launch_bounds__(kHeatMaxTile / 8, 8)
-    k_swept_heat4(const Params<float> p, float *__restrict__ state, float *__restrict__ slots, const int W, const int phase) {
+    k_swept_heat4(const Params<float> p, float *state, float *slots, const int W, const int phase) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     float *rows = reinterpret_cast<float *>(sw_smem);
     wait_for_previous_launch();
