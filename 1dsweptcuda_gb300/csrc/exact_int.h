@@ -95,8 +95,8 @@ SW_HD double mul6(double x) {
 
 // ---- general products, quotients and square roots on the integer pipe
 //
-// mul_int_fast(x, y, bad) = x * y, div_int_fast(x, y, bad) = x / y and
-// sqrt_int_fast(x, bad) = sqrt(x), each rounded once (to nearest, ties to
+// mul_int_fast(x, y, bad) = x * y, div_int_with(x, rcp_int(y), bad) = x / y
+// and sqrt_int_fast(x, bad) = sqrt(x), each rounded once (to nearest, ties to
 // even), for normal operands with a normal result (biased exponent at most
 // 2045 before rounding); a division also takes a zero numerator.  For
 // anything else -- other zeros, subnormals, infinities, NaNs, a result near or
@@ -292,7 +292,6 @@ SW_HD double div_int_with(double a, const RcpInt &b, uint32_t &bad) {
     bad |= (uint32_t)!(eb - 1u < 2046u && (zero || (ea - 1u < 2046u && ea - eb + 1021u + top < 2045u)));
     return f64_of(zero ? sgn : ((e + mh) | sgn), zero ? 0u : ml);
 }
-SW_HD double div_int_fast(double a, double b, uint32_t &bad) { return div_int_with(a, rcp_int(b), bad); }
 
 // ---- square roots
 //

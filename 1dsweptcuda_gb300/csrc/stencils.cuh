@@ -89,7 +89,9 @@ SW_HD double half_min1(double r) { return half_min1_any(r); }
 SW_HD float half_min1(float r) { return ml(mn(r, 1.0f), 0.5f); }
 SW_HD bool is_zero(float x) { return x == 0.0f; }
 SW_HD bool is_neg(float x) { return x < 0.0f; }
-// b - a from d = a - b: -d, but equal values differ by +0 both ways
+// b - a from d = a - b: -d, but equal values differ by +0 both ways.  Zeros of
+// opposite signs do not: a = +0, b = -0 gives d = +0 and here +0 for -0.  Its
+// user adds a multiple of the result to a, and +0 plus a zero of either sign is +0.
 SW_HD double neg_diff(double d) { return f64_from_bits(f64_bits(d) == 0 ? 0 : f64_bits(d) ^ 0x8000000000000000ull); }
 SW_HD float neg_diff(float d) { return d == 0.0f ? 0.0f : -d; }
 // a product on the integer pipe (INT) or the FP64 pipe

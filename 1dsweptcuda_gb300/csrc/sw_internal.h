@@ -96,8 +96,13 @@ struct Ops {
 // cells 1.5 and 4.8 against 1.8 and 5.0, 512 cells 0.9 and 3.1; KS FP32 128 cells
 // 3.0 and 9.3 against 4.1 and 10.9, 512 cells 1.9 and 6.1; Heat FP64 128 cells 6.3
 // and 24 against 7.3 and 25.  64 cells lose there (Heat FP32 2.8 and 10), but not
-// on small domains (4096 cells: 0.8 against 1.7).  FP64 KS and Euler are bound by
-// arithmetic, which classic wastes none of (KS FP64 128 cells 52 against 49).
+// on small domains (4096 cells: 0.8 against 1.7).  Euler takes none: the steps left
+// over ran 0.4x to 1.0x as fast in narrow cycles, FP32 and FP64, 2^10 to 2^20 cells,
+// tiles 128 to 1024.  FP64 KS takes none either: on large domains it is bound by
+// arithmetic, which classic wastes none of (2^20 cells, tile 256, 31 steps: 1608 us
+// against 1565).  On small ones launches bound it as they do the others, and narrow
+// cycles would be the faster ones: 31 steps of tile 256 at 2^12 cells 141 against 173,
+// 127 of tile 1024 585 against 1258, at 2^18 cells 2013 against 2162.
 inline int tail_tile(const Ops &ops, bool divide, int W, int64_t cells, int64_t rem) {
     if (divide || ops.problem == SW_EULER || (ops.problem == SW_KS && ops.prec == 8)) return 0;
     const int least = cells <= ((int64_t)1 << 18) ? 64 : 128;

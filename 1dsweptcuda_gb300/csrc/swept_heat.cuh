@@ -234,8 +234,11 @@ __global__ void __launch_bounds__(kHeatMaxTile / 8, 8)
 // per SM.  us for W cells per tile, insulated ends, 4 cycles (2 at 2^20 cells and above), tile_span4 -> here: 2^22 cells
 // 192 877 -> 609, 256 922 -> 621, 512 1637 -> 1117, 768 2320 -> 1284, 1024 2971 -> 1619 (1.30e12 -> 2.36e12
 // cell-updates/s); 2^18 cells 192 223 -> 216, 256 287 -> 238, 512 402 -> 386, 1024 731 -> 677; 2^12 cells 192 176 -> 181,
-// 256 209 -> 217, 512 345 -> 349, 768 506 -> 484, 1024 668 -> 615.  Narrower tiles (equal at 128 and 64, 0.8x at 32) and
-// part-empty warps (384: 0.9x at 2^18) keep tile_span4.
+// 256 209 -> 217, 512 345 -> 349, 768 506 -> 484, 1024 668 -> 615.  Narrower tiles (equal at 128 and 64, 0.8x at 32) keep
+// tile_span4, and so do the widths above 256 that leave a part-empty warp.  Of those only the narrow ones on 2^18 cells
+// lose here (288 to 416 cells, 0.91x to 0.95x); us, tile_span4 -> here, 4 cycles at 2^18 cells, 2 at 2^20 and 2^22: 384
+// 313 -> 340, 394 -> 353, 1294 -> 1090; 640 463 -> 438, 583 -> 429, 1997 -> 1189; 896 624 -> 575, 787 -> 484, 2654 ->
+// 1525.  The line is not at that crossover yet.
 inline bool heat4_tiles(int W, int64_t ntile) {
     if (W > kHeatMaxTile || (W % 256 != 0 && (W < 192 || W > 256))) return false;
     return W >= 768 || !few_tiles(ntile);
